@@ -20,6 +20,7 @@
 #include <unordered_map>
 
 #include "born_kernels.cuh"
+#include "chain2d.cuh"
 #include "devbuf.hpp"
 #include "geometry.cuh"
 #include "gmres_kernels.cuh"
@@ -89,6 +90,9 @@ class PlaneSolver final : public Solver {
   // the forward/backward sweeps of a run (device work only, unless Born slabs need GMRES)
   void sweeps(int iterations, const std::vector<int>& keep_slot, DevBuf<C>& kept_f, DevBuf<C>& kept_b,
               DevBuf<C>& t_iter, DevBuf<C>& r_iter);
+  // the sweeps of a 2D run without Born slabs, as one launch (chain2d.cuh)
+  void chain(int iterations, const std::vector<int>& keep_slot, bool any_keep, DevBuf<C>& kept_f,
+             DevBuf<C>& kept_b, DevBuf<C>& t_iter, DevBuf<C>& r_iter);
   void axpby(C* y, const C* x, cd a, cd b, long long m);
   void add_plane_scaled(C* dst, const C* src, const T* mask);
   LaunchShape rows_shape(int ncomp, int rows_max) const;
@@ -143,6 +147,11 @@ class PlaneSolver final : public Solver {
   // launch shapes
   int thr2d_ = 32, thr_line3_ = 32;
   bool line_ept8_ = false;  // 2D line transforms with 8 values per thread (k_line_fft)
+  // 2D without Born slabs: one launch runs all sweeps (fn null: a launch per step instead)
+  ChainKernel chain_;
+  HostPlan chain_plan_;
+  DevBuf<Tw<T>> tw_chain_;
+  DevBuf<R2Step> chain_steps_;
   int sms_ = 148;
   LaunchShape rows2_, rows3_, sel_, cols1_, cols2_, cols3_;
   std::int64_t launches_ = 0, gmres_applies_ = 0;
@@ -474,6 +483,16 @@ void PlaneSolver<T>::setup() {
     for (auto k : {(const void*)k_line_fft<-1, T>, (const void*)k_line_fft<1, T>,
                    (const void*)k_line_fft<-1, T, 8>, (const void*)k_line_fft<1, T, 8>})
       check_cuda(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024), "smem");
+    // BWPM_2D_KERNELS=step selects the launch-per-step form
+    const char* k2 = std::getenv("BWPM_2D_KERNELS");
+    if (hosts_.empty() && in_.nz > 0 && !(k2 && std::strcmp(k2, "step") == 0))
+      chain_ = chain_kernel<T>(static_cast<int>(in_.ny), !in_.mask.empty());
+    if (chain_.fn) {
+      chain_plan_ = make_plan_radices(static_cast<int>(in_.ny), chain_.radices);
+      upload_tw(chain_plan_, tw_chain_);
+      check_cuda(cudaFuncSetAttribute(chain_.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(chain_.smem)), "smem");
+    }
   } else {
     rows2_ = rows_shape(2, 8);
     rows3_ = rows_shape(3, 8);
@@ -726,7 +745,56 @@ void PlaneSolver<T>::ensure_passes(bool with_backward) {
   }
   pass_pool_.alloc(host.size(), stream_);
   pass_pool_.upload(host.data(), host.size());
+  if (chain_.fn) {
+    std::vector<R2Step> recs(in_.nz);
+    for (std::size_t s = 0; s < in_.nz; ++s)
+      recs[s] = {steps_[s].pid_off, steps_[s].iface_off, steps_[s].niface,
+                 static_cast<int>(pass_off_[0][s]), pass_nt_[0][s], pass_nr_[0][s],
+                 static_cast<int>(pass_off_[1][s]), pass_nt_[1][s], pass_nr_[1][s]};
+    chain_steps_.alloc(recs.size(), stream_);
+    chain_steps_.upload(recs.data(), recs.size());
+  }
   pool_dirs_ = dirs;
+}
+
+template <typename T>
+void PlaneSolver<T>::chain(int iterations, const std::vector<int>& keep_slot, bool any_keep,
+                           DevBuf<C>& kept_f, DevBuf<C>& kept_b, DevBuf<C>& t_iter,
+                           DevBuf<C>& r_iter) {
+  DevBuf<int> keep;
+  if (any_keep) {
+    keep.alloc(keep_slot.size(), stream_);
+    keep.upload(keep_slot.data(), keep_slot.size());
+  }
+  ChainArgs<T> a;
+  a.input = input_.ptr;
+  a.t_out = iterations > 0 ? t_iter.ptr : e_.ptr;
+  a.r_out = r_iter.ptr;
+  a.kept_f = kept_f.ptr;
+  a.kept_b = kept_b.ptr;
+  a.keep = keep.ptr;
+  a.steps = chain_steps_.ptr;
+  a.passes = pass_pool_.ptr;
+  a.pids = pid_pool_.ptr;
+  a.iface = iface_pool_.ptr;
+  a.src_fwd = src_fwd_.ptr;
+  a.src_bwd = src_bwd_.ptr;
+  a.mask = mask_.ptr;
+  a.spec = spec_.ptr;
+  a.tw = tw_chain_.ptr;
+  a.n = static_cast<int>(n());
+  a.nz = static_cast<int>(in_.nz);
+  a.iterations = iterations;
+  a.ntw = static_cast<int>(n()) - 1;
+  a.tw_smem = chain_.tw_smem;
+  a.mask_smem = chain_.mask_smem;
+  a.spec_smem = chain_.spec_smem;
+  a.inv_n = sizeof(T) == sizeof(double) ? static_cast<T>(1.0 / static_cast<double>(n())) : T(1);
+  void* args[] = {&a, &chain_plan_.plan};
+  check_cuda(cudaLaunchKernel(chain_.fn, dim3(2), dim3(chain_.threads), args, chain_.smem, stream_),
+             "k_chain2d");
+  ++launches_;
+  last_e_ = e_.ptr;
 }
 
 template <typename T>
@@ -1263,7 +1331,10 @@ void PlaneSolver<T>::run(const cd* field, int iterations, const std::int64_t* ke
   check_cuda(cudaMemcpyAsync(stage_.ptr, field, n2 * sizeof(cd), cudaMemcpyHostToDevice, stream_), "field upload");
   launch(k_convert<T, double>, dim3(ceil_div(n2, kThreads)), dim3(kThreads), 0, input_.ptr,
          (const cd*)stage_.ptr, n2);
-  sweeps(iterations, keep_slot, kept_f, kept_b, t_iter, r_iter);
+  if (chain_.fn)
+    chain(iterations, keep_slot, nkeep > 0, kept_f, kept_b, t_iter, r_iter);
+  else
+    sweeps(iterations, keep_slot, kept_f, kept_b, t_iter, r_iter);
   C* e = last_e_;
   // outputs
   auto download = [&](const C* src, cd* dst) {

@@ -1,4 +1,5 @@
-// Register-resident FFT for lines of a compile-time length N (complex64, split constants).
+// Register-resident FFT for lines of a compile-time length N (complex64 with split constants, or
+// FP64).
 //
 // NT threads, E = N/NT values per thread. Thread t owns positions t + m·NT (m < E): the
 // "owned pattern". In the Stockham stage of radix R (sub-length L) the thread's butterflies are
@@ -11,8 +12,8 @@
 // power-of-two stride and the owned reads free of bank conflicts.
 //
 // Twiddles: the per-stage r-major tables of plan.hpp (entry (r − 1)·L + k of stage s at offset
-// Σ_{s'<s} L_s'·(R_s' − 1)), stored as FP32 (hi, lo) pairs; see fft.cuh for why every constant is
-// carried as a pair.
+// Σ_{s'<s} L_s'·(R_s' − 1)), stored as FP32 (hi, lo) pairs or FP64 values; see fft.cuh for why every
+// FP32 constant is carried as a pair.
 #pragma once
 
 #include "fft.cuh"
@@ -23,8 +24,12 @@ namespace rf {
 template <int... Rs>
 struct Radices {};
 
-__device__ __forceinline__ int pad(int a) { return a + (a >> 4); }
-__host__ __device__ constexpr int padded(int n) { return n + n / 16 + 1; }
+// Padding by the element's size: FP32 complex values (8 bytes) one element per 16, FP64 ones
+// (16 bytes: a quarter warp covers the banks) one per 8.
+template <typename T = float>
+__device__ __forceinline__ int pad(int a) { return a + (a >> (sizeof(T) == sizeof(double) ? 3 : 4)); }
+template <typename T = float>
+__host__ __device__ constexpr int padded(int n) { return n + n / (sizeof(T) == sizeof(double) ? 8 : 16) + 1; }
 
 // x·exp(DIR·2πi·e/16) with exact (±1, ±i) cases and split constants otherwise.
 template <int DIR, int EXP>
@@ -89,18 +94,97 @@ __device__ __forceinline__ void dft16(cf* u) {
   }
 }
 
-template <int DIR, int R>
-__device__ __forceinline__ void dft(cf* u) {
+// x·(c ± i·s) for a constant c + i·s (FP32: split).
+template <int DIR, typename T>
+__device__ __forceinline__ cx<T> cmulk(cx<T> x, double c, double s) {
+  const double si = DIR * s;
+  if constexpr (sizeof(T) == sizeof(double)) {
+    return {fma(x.re, c, -x.im * si), fma(x.re, si, x.im * c)};
+  } else {
+    const cf hi{static_cast<float>(c), static_cast<float>(si)};
+    const cf lo{static_cast<float>(c - static_cast<double>(hi.re)),
+                static_cast<float>(si - static_cast<double>(hi.im))};
+    return pmul(x, hi, lo);
+  }
+}
+
+// Radix 9 as 3 × 3: n = 3·n1 + n2, m = m1 + 3·m2, twiddles w9^(n2·m1) (cosines and sines of
+// 40°, 80° and 160°).
+template <int DIR, typename T>
+__device__ __forceinline__ void dft9(cx<T>* u) {
+  constexpr double c1 = 0.76604444311897803520, s1 = 0.64278760968653932632;
+  constexpr double c2 = 0.17364817766693034885, s2 = 0.98480775301220805937;
+  constexpr double c4 = -0.93969262078590838405, s4 = 0.34202014332566873304;
+  cx<T> a[3][3];
+#pragma unroll
+  for (int n2 = 0; n2 < 3; ++n2) {
+#pragma unroll
+    for (int n1 = 0; n1 < 3; ++n1) a[n2][n1] = u[3 * n1 + n2];
+    fftdetail::dft3<DIR>(a[n2]);
+  }
+  a[1][1] = cmulk<DIR>(a[1][1], c1, s1);
+  a[1][2] = cmulk<DIR>(a[1][2], c2, s2);
+  a[2][1] = cmulk<DIR>(a[2][1], c2, s2);
+  a[2][2] = cmulk<DIR>(a[2][2], c4, s4);
+#pragma unroll
+  for (int m1 = 0; m1 < 3; ++m1) {
+    cx<T> b[3] = {a[0][m1], a[1][m1], a[2][m1]};
+    fftdetail::dft3<DIR>(b);
+#pragma unroll
+    for (int m2 = 0; m2 < 3; ++m2) u[m1 + 3 * m2] = b[m2];
+  }
+}
+
+// Radix A·B of coprime A, B without twiddles (prime-factor map, I. J. Good 1958): inputs
+// n = B·n1 + A·n2, outputs k ≡ k1 (mod A), k2 (mod B).
+__host__ __device__ constexpr int pfa_out(int k1, int k2, int A, int B) {
+  for (int k = 0; k < A * B; ++k)
+    if (k % A == k1 && k % B == k2) return k;
+  return 0;
+}
+template <int DIR, int A, int B, typename T>
+__device__ __forceinline__ void dft_pfa(cx<T>* u) {
+  cx<T> a[B][A];
+#pragma unroll
+  for (int n2 = 0; n2 < B; ++n2) {
+#pragma unroll
+    for (int n1 = 0; n1 < A; ++n1) a[n2][n1] = u[(B * n1 + A * n2) % (A * B)];
+    fftdetail::dft<DIR, A>(a[n2]);
+  }
+#pragma unroll
+  for (int k1 = 0; k1 < A; ++k1) {
+    cx<T> b[B];
+#pragma unroll
+    for (int n2 = 0; n2 < B; ++n2) b[n2] = a[n2][k1];
+    fftdetail::dft<DIR, B>(b);
+#pragma unroll
+    for (int k2 = 0; k2 < B; ++k2) u[pfa_out(k1, k2, A, B)] = b[k2];
+  }
+}
+
+template <int DIR, int R, typename T>
+__device__ __forceinline__ void dft(cx<T>* u) {
+  static_assert(R != 16 || sizeof(T) == sizeof(float), "radix 16 is FP32 only");
   if constexpr (R == 16)
     dft16<DIR>(u);
+  else if constexpr (R == 6)
+    dft_pfa<DIR, 2, 3>(u);
+  else if constexpr (R == 9)
+    dft9<DIR>(u);
+  else if constexpr (R == 10)
+    dft_pfa<DIR, 2, 5>(u);
+  else if constexpr (R == 12)
+    dft_pfa<DIR, 3, 4>(u);
+  else if constexpr (R == 15)
+    dft_pfa<DIR, 3, 5>(u);
   else
     fftdetail::dft<DIR, R>(u);
 }
 
 // One stage; v holds the owned values on entry (stage input) and on exit (next stage's input,
 // or the transform's output after the last stage).
-template <int DIR, int N, int NT, int R, int L, int OFF, bool LAST>
-__device__ __forceinline__ void stage(cf (&v)[N / NT], cf* buf, const Tw<float>* __restrict__ tw,
+template <int DIR, int N, int NT, int R, int L, int OFF, bool LAST, typename T>
+__device__ __forceinline__ void stage(cx<T> (&v)[N / NT], cx<T>* buf, const Tw<T>* __restrict__ tw,
                                       int t) {
   constexpr int E = N / NT, K = E / R;
   static_assert(E % R == 0, "radix must divide the values per thread");
@@ -108,7 +192,7 @@ __device__ __forceinline__ void stage(cf (&v)[N / NT], cf* buf, const Tw<float>*
   for (int j = 0; j < K; ++j) {
     const int i = t + j * NT;
     const int k = i % L;
-    cf u[R];
+    cx<T> u[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) u[r] = v[j + r * K];
     if constexpr (L > 1) {
@@ -122,7 +206,7 @@ __device__ __forceinline__ void stage(cf (&v)[N / NT], cf* buf, const Tw<float>*
     } else {
       const int base = (i - k) * R + k;
 #pragma unroll
-      for (int r = 0; r < R; ++r) buf[pad(base + r * L)] = u[r];
+      for (int r = 0; r < R; ++r) buf[pad<T>(base + r * L)] = u[r];
     }
     // compiler-only fence: one butterfly's twiddles and temporaries are dead before the next
     // butterfly's loads are issued (keeps the live registers of a stage at one butterfly)
@@ -131,7 +215,7 @@ __device__ __forceinline__ void stage(cf (&v)[N / NT], cf* buf, const Tw<float>*
   if constexpr (!LAST) {
     __syncthreads();
 #pragma unroll
-    for (int m = 0; m < E; ++m) v[m] = buf[pad(t + m * NT)];
+    for (int m = 0; m < E; ++m) v[m] = buf[pad<T>(t + m * NT)];
   }
 }
 
@@ -139,21 +223,21 @@ __device__ __forceinline__ void stage(cf (&v)[N / NT], cf* buf, const Tw<float>*
 // each thread gathers whole butterflies i = t + j·NT < N/R (the last round partly idle), writes
 // their outputs to out_buf and reads back its owned values. Two barriers instead of one; the
 // caller leaves `phase` as it was (both buffers were used, the last reads were from out_buf).
-template <int DIR, int N, int NT, int R, int L, int OFF>
-__device__ __forceinline__ void stage_gather(cf (&v)[N / NT], cf* in_buf, cf* out_buf,
-                                             const Tw<float>* __restrict__ tw, int t) {
+template <int DIR, int N, int NT, int R, int L, int OFF, typename T>
+__device__ __forceinline__ void stage_gather(cx<T> (&v)[N / NT], cx<T>* in_buf, cx<T>* out_buf,
+                                             const Tw<T>* __restrict__ tw, int t) {
   constexpr int E = N / NT, NB = N / R, KG = (NB + NT - 1) / NT;
 #pragma unroll
-  for (int m = 0; m < E; ++m) in_buf[pad(t + m * NT)] = v[m];
+  for (int m = 0; m < E; ++m) in_buf[pad<T>(t + m * NT)] = v[m];
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < KG; ++j) {
     const int i = t + j * NT;
     if (NB % NT == 0 || i < NB) {
       const int k = i % L;
-      cf u[R];
+      cx<T> u[R];
 #pragma unroll
-      for (int r = 0; r < R; ++r) u[r] = in_buf[pad(i + r * NB)];
+      for (int r = 0; r < R; ++r) u[r] = in_buf[pad<T>(i + r * NB)];
       if constexpr (L > 1) {
 #pragma unroll
         for (int r = 1; r < R; ++r) u[r] = twmul<DIR>(u[r], tw[OFF + (r - 1) * L + k]);
@@ -161,18 +245,18 @@ __device__ __forceinline__ void stage_gather(cf (&v)[N / NT], cf* in_buf, cf* ou
       dft<DIR, R>(u);
       const int base = (i - k) * R + k;
 #pragma unroll
-      for (int r = 0; r < R; ++r) out_buf[pad(base + r * L)] = u[r];
+      for (int r = 0; r < R; ++r) out_buf[pad<T>(base + r * L)] = u[r];
     }
     asm volatile("" ::: "memory");
   }
   __syncthreads();
 #pragma unroll
-  for (int m = 0; m < E; ++m) v[m] = out_buf[pad(t + m * NT)];
+  for (int m = 0; m < E; ++m) v[m] = out_buf[pad<T>(t + m * NT)];
 }
 
-template <int DIR, int N, int NT, int L, int OFF, int R, int... Rest>
-__device__ __forceinline__ void stages(cf (&v)[N / NT], cf* b0, cf* b1, int& phase,
-                                       const Tw<float>* __restrict__ tw, int t) {
+template <int DIR, int N, int NT, int L, int OFF, int R, int... Rest, typename T>
+__device__ __forceinline__ void stages(cx<T> (&v)[N / NT], cx<T>* b0, cx<T>* b1, int& phase,
+                                       const Tw<T>* __restrict__ tw, int t) {
   constexpr bool last = sizeof...(Rest) == 0;
   if constexpr ((N / NT) % R == 0) {
     stage<DIR, N, NT, R, L, OFF, last>(v, phase ? b1 : b0, tw, t);
@@ -186,11 +270,77 @@ __device__ __forceinline__ void stages(cf (&v)[N / NT], cf* b0, cf* b1, int& pha
 // In-register transform of the owned values (DIR −1 forward, +1 inverse unnormalised).
 // `phase` selects the exchange buffer and must be uniform across the block; the buffer it
 // points to after the transform is free for the caller (no thread still reads it).
-template <int DIR, int N, int NT, int... Rs>
-__device__ __forceinline__ void fft(cf (&v)[N / NT], cf* b0, cf* b1, int& phase,
-                                   const Tw<float>* __restrict__ tw, int t, Radices<Rs...>) {
+template <int DIR, int N, int NT, int... Rs, typename T>
+__device__ __forceinline__ void fft(cx<T> (&v)[N / NT], cx<T>* b0, cx<T>* b1, int& phase,
+                                   const Tw<T>* __restrict__ tw, int t, Radices<Rs...>) {
   static_assert((1 * ... * Rs) == N, "radices must multiply to N");
   stages<DIR, N, NT, 1, 0, Rs...>(v, b0, b1, phase, tw, t);
+}
+
+// ---- transforms whose inner stages take any radix -----------------------------------------------
+//
+// The first and the last stage's radix divides E, so the transform still goes registers to
+// registers in the owned pattern; every stage between reads whole butterflies i = t + j·NT < N/R
+// from the exchange buffer that the stage before wrote and writes the other one: one exchange and
+// one barrier per stage boundary for any inner radix (stage_gather takes two exchanges). With the
+// composite radices 6, 9, 10, 12 and 15 a 3·2^k or 5-smooth line needs as few stages as a power
+// of two (384 = 8·6·8, 3072 = 8·8·6·8, 2430 = 9·5·6·9).
+
+template <int DIR, int N, int NT, int R, int L, int OFF, bool FIRST, bool LAST, typename T>
+__device__ __forceinline__ void gstage(cx<T> (&v)[N / NT], const cx<T>* in_buf, cx<T>* out_buf,
+                                       const Tw<T>* __restrict__ tw, int t) {
+  constexpr int E = N / NT, NB = N / R, KG = (NB + NT - 1) / NT, K = FIRST || LAST ? E / R : 1;
+  static_assert(!(FIRST || LAST) || E % R == 0, "the outer radices must divide the values per thread");
+#pragma unroll
+  for (int j = 0; j < KG; ++j) {
+    const int i = t + j * NT;
+    if (NB % NT == 0 || i < NB) {
+      const int k = i % L;
+      cx<T> u[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        if constexpr (FIRST)
+          u[r] = v[j + r * K];
+        else
+          u[r] = in_buf[pad<T>(i + r * NB)];
+      }
+      if constexpr (L > 1) {
+#pragma unroll
+        for (int r = 1; r < R; ++r) u[r] = twmul<DIR>(u[r], tw[OFF + (r - 1) * L + k]);
+      }
+      dft<DIR, R>(u);
+      if constexpr (LAST) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[j + r * K] = u[r];
+      } else {
+        const int base = (i - k) * R + k;
+#pragma unroll
+        for (int r = 0; r < R; ++r) out_buf[pad<T>(base + r * L)] = u[r];
+      }
+    }
+    asm volatile("" ::: "memory");
+  }
+  if constexpr (!LAST) __syncthreads();
+}
+
+template <int DIR, int N, int NT, int L, int OFF, bool FIRST, int R, int... Rest, typename T>
+__device__ __forceinline__ void gstages(cx<T> (&v)[N / NT], cx<T>* b0, cx<T>* b1, int& phase,
+                                        const Tw<T>* __restrict__ tw, int t) {
+  constexpr bool last = sizeof...(Rest) == 0;
+  // reads the buffer written by the stage before (phase ^ 1), writes buffer `phase`
+  gstage<DIR, N, NT, R, L, OFF, FIRST, last>(v, phase ? b0 : b1, phase ? b1 : b0, tw, t);
+  if constexpr (!last) {
+    phase ^= 1;
+    gstages<DIR, N, NT, L * R, OFF + L * (R - 1), false, Rest...>(v, b0, b1, phase, tw, t);
+  }
+}
+
+// As fft(), with any inner radices.
+template <int DIR, int N, int NT, int... Rs, typename T>
+__device__ __forceinline__ void gfft(cx<T> (&v)[N / NT], cx<T>* b0, cx<T>* b1, int& phase,
+                                     const Tw<T>* __restrict__ tw, int t, Radices<Rs...>) {
+  static_assert((1 * ... * Rs) == N, "radices must multiply to N");
+  gstages<DIR, N, NT, 1, 0, true, Rs...>(v, b0, b1, phase, tw, t);
 }
 
 }  // namespace rf

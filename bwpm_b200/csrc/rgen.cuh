@@ -16,8 +16,8 @@
 namespace bwpm {
 namespace rg {
 
-template <int DIR, int E, int R>
-__device__ __forceinline__ void stage(cf (&v)[E], cf* buf, const Tw<float>* __restrict__ tw, int t,
+template <int DIR, int E, int R, typename T>
+__device__ __forceinline__ void stage(cx<T> (&v)[E], cx<T>* buf, const Tw<T>* __restrict__ tw, int t,
                                       int nt, int L, int off, bool last) {
   constexpr int K = E / R;
   static_assert(E % R == 0, "radix must divide the values per thread");
@@ -26,7 +26,7 @@ __device__ __forceinline__ void stage(cf (&v)[E], cf* buf, const Tw<float>* __re
     for (int j = 0; j < K; ++j) {
       const int i = t + j * nt;
       const int k = i % L;
-      cf u[R];
+      cx<T> u[R];
 #pragma unroll
       for (int r = 0; r < R; ++r) u[r] = v[j + r * K];
       if (L > 1) {
@@ -40,7 +40,7 @@ __device__ __forceinline__ void stage(cf (&v)[E], cf* buf, const Tw<float>* __re
       } else {
         const int base = (i - k) * R + k;
 #pragma unroll
-        for (int r = 0; r < R; ++r) buf[rf::pad(base + r * L)] = u[r];
+        for (int r = 0; r < R; ++r) buf[rf::pad<T>(base + r * L)] = u[r];
       }
       asm volatile("" ::: "memory");
     }
@@ -49,7 +49,7 @@ __device__ __forceinline__ void stage(cf (&v)[E], cf* buf, const Tw<float>* __re
     __syncthreads();
     if (t < nt) {
 #pragma unroll
-      for (int m = 0; m < E; ++m) v[m] = buf[rf::pad(t + m * nt)];
+      for (int m = 0; m < E; ++m) v[m] = buf[rf::pad<T>(t + m * nt)];
     }
   }
 }
@@ -58,21 +58,21 @@ __device__ __forceinline__ void stage(cf (&v)[E], cf* buf, const Tw<float>* __re
 // gathers whole butterflies (i = t + j·nt < n/R, a run-time count), writes the outputs to the
 // other buffer, and reads back its owned values. Two barriers instead of one; `phase` is left
 // as it was (both buffers were used, the last reads were from the other one).
-template <int DIR, int E, int R>
-__device__ __forceinline__ void stage_gather(cf (&v)[E], cf* in_buf, cf* out_buf,
-                                             const Tw<float>* __restrict__ tw, int t, int nt, int n,
+template <int DIR, int E, int R, typename T>
+__device__ __forceinline__ void stage_gather(cx<T> (&v)[E], cx<T>* in_buf, cx<T>* out_buf,
+                                             const Tw<T>* __restrict__ tw, int t, int nt, int n,
                                              int L, int off) {
   if (t < nt) {
 #pragma unroll
-    for (int m = 0; m < E; ++m) in_buf[rf::pad(t + m * nt)] = v[m];
+    for (int m = 0; m < E; ++m) in_buf[rf::pad<T>(t + m * nt)] = v[m];
   }
   __syncthreads();
   const int nb = n / R;
   for (int i = t; i < nb; i += nt) {
     const int k = i % L;
-    cf u[R];
+    cx<T> u[R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) u[r] = in_buf[rf::pad(i + r * nb)];
+    for (int r = 0; r < R; ++r) u[r] = in_buf[rf::pad<T>(i + r * nb)];
     if (L > 1) {
 #pragma unroll
       for (int r = 1; r < R; ++r) u[r] = twmul<DIR>(u[r], tw[off + (r - 1) * L + k]);
@@ -80,20 +80,20 @@ __device__ __forceinline__ void stage_gather(cf (&v)[E], cf* in_buf, cf* out_buf
     rf::dft<DIR, R>(u);
     const int base = (i - k) * R + k;
 #pragma unroll
-    for (int r = 0; r < R; ++r) out_buf[rf::pad(base + r * L)] = u[r];
+    for (int r = 0; r < R; ++r) out_buf[rf::pad<T>(base + r * L)] = u[r];
   }
   __syncthreads();
   if (t < nt) {
 #pragma unroll
-    for (int m = 0; m < E; ++m) v[m] = out_buf[rf::pad(t + m * nt)];
+    for (int m = 0; m < E; ++m) v[m] = out_buf[rf::pad<T>(t + m * nt)];
   }
 }
 
 // In-register transform (DIR −1 forward, +1 inverse unnormalised) of a line of E·nt points with
 // the stages of `plan`; `phase` as in rf::fft. Every thread of the block must call it.
-template <int DIR, int E, int R>
-__device__ __forceinline__ void any_stage(cf (&v)[E], cf* b0, cf* b1, int& phase,
-                                          const Tw<float>* __restrict__ tw, int t, int nt, int n,
+template <int DIR, int E, int R, typename T>
+__device__ __forceinline__ void any_stage(cx<T> (&v)[E], cx<T>* b0, cx<T>* b1, int& phase,
+                                          const Tw<T>* __restrict__ tw, int t, int nt, int n,
                                           int L, int off, bool last) {
   if constexpr (E % R == 0) {
     stage<DIR, E, R>(v, phase ? b1 : b0, tw, t, nt, L, off, last);
@@ -103,9 +103,9 @@ __device__ __forceinline__ void any_stage(cf (&v)[E], cf* b0, cf* b1, int& phase
   }
 }
 
-template <int DIR, int E>
-__device__ __forceinline__ void fft(cf (&v)[E], cf* b0, cf* b1, int& phase, const FftPlan& plan,
-                                   const Tw<float>* __restrict__ tw, int t, int nt) {
+template <int DIR, int E, typename T>
+__device__ __forceinline__ void fft(cx<T> (&v)[E], cx<T>* b0, cx<T>* b1, int& phase, const FftPlan& plan,
+                                   const Tw<T>* __restrict__ tw, int t, int nt) {
   for (int s = 0; s < plan.nstages; ++s) {
     const bool last = s == plan.nstages - 1;
     const int L = plan.len[s], off = plan.twoff[s];
@@ -117,6 +117,84 @@ __device__ __forceinline__ void fft(cf (&v)[E], cf* b0, cf* b1, int& phase, cons
       case 8: any_stage<DIR, E, 8>(v, b0, b1, phase, tw, t, nt, plan.n, L, off, last); break;
       default: break;  // the host plans radices 2, 3, 4, 5 and 8 only
     }
+  }
+}
+
+// ---- run-time lengths with equal outer radices --------------------------------------------------
+//
+// The transform of rf::gfft for a run-time length n = E·nt: the first and the last stage have
+// radix E (the owned pattern), the stages between any radix of gmid, chosen by the host
+// (chain2d.cuh); one exchange per stage boundary.
+
+// i mod L for i < 2^15 by a multiplication with ⌈2^32/L⌉ (exact: i·L < 2^32).
+__device__ __forceinline__ int mod_magic(int i, int L, unsigned magic) {
+  return i - static_cast<int>(__umulhi(static_cast<unsigned>(i), magic)) * L;
+}
+
+// An inner stage of radix R over all threads of the block.
+template <int DIR, int R, typename T>
+__device__ __forceinline__ void gmid(const cx<T>* in_buf, cx<T>* out_buf,
+                                     const Tw<T>* __restrict__ tw, int n, int L, unsigned magic) {
+  const int nb = n / R;
+  for (int i = threadIdx.x; i < nb; i += static_cast<int>(blockDim.x)) {
+    const int k = mod_magic(i, L, magic);
+    cx<T> u[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) u[r] = in_buf[rf::pad<T>(i + r * nb)];
+#pragma unroll
+    for (int r = 1; r < R; ++r) u[r] = twmul<DIR>(u[r], tw[(r - 1) * L + k]);
+    rf::dft<DIR, R>(u);
+    const int base = (i - k) * R + k;
+#pragma unroll
+    for (int r = 0; r < R; ++r) out_buf[rf::pad<T>(base + r * L)] = u[r];
+  }
+}
+
+// In-register transform of a line of n = E·nt points, plan radices (E, inner …, E); `phase` as
+// in rf::fft. Every thread of the block must call it; magic[s] belongs to plan.len[s].
+template <int DIR, int E, typename T>
+__device__ __forceinline__ void gfft(cx<T> (&v)[E], cx<T>* b0, cx<T>* b1, int& phase, const FftPlan& plan,
+                                     const unsigned* magic, const Tw<T>* __restrict__ tw, int t,
+                                     int nt) {
+  const bool own = t < nt;
+  {  // first stage: butterfly t of radix E, sub-length 1
+    if (own) {
+      cx<T>* out = phase ? b1 : b0;
+      rf::dft<DIR, E>(v);
+#pragma unroll
+      for (int r = 0; r < E; ++r) out[rf::pad<T>(t * E + r)] = v[r];
+    }
+    __syncthreads();
+    phase ^= 1;
+  }
+  for (int s = 1; s + 1 < plan.nstages; ++s) {
+    const cx<T>* in = phase ? b0 : b1;
+    cx<T>* out = phase ? b1 : b0;
+    const int L = plan.len[s];
+    const Tw<T>* w = tw + plan.twoff[s];
+    switch (plan.radix[s]) {
+      case 2: gmid<DIR, 2>(in, out, w, plan.n, L, magic[s]); break;
+      case 3: gmid<DIR, 3>(in, out, w, plan.n, L, magic[s]); break;
+      case 4: gmid<DIR, 4>(in, out, w, plan.n, L, magic[s]); break;
+      case 5: gmid<DIR, 5>(in, out, w, plan.n, L, magic[s]); break;
+      case 6: gmid<DIR, 6>(in, out, w, plan.n, L, magic[s]); break;
+      case 7: gmid<DIR, 7>(in, out, w, plan.n, L, magic[s]); break;
+      case 8: gmid<DIR, 8>(in, out, w, plan.n, L, magic[s]); break;
+      case 9: gmid<DIR, 9>(in, out, w, plan.n, L, magic[s]); break;
+      case 10: gmid<DIR, 10>(in, out, w, plan.n, L, magic[s]); break;
+      default: break;  // the host plans inner radices 2 to 10 only
+    }
+    __syncthreads();
+    phase ^= 1;
+  }
+  if (own) {  // last stage: sub-length nt, butterfly t
+    const cx<T>* in = phase ? b0 : b1;
+    const Tw<T>* w = tw + plan.twoff[plan.nstages - 1];
+#pragma unroll
+    for (int r = 0; r < E; ++r) v[r] = in[rf::pad<T>(t + r * nt)];
+#pragma unroll
+    for (int r = 1; r < E; ++r) v[r] = twmul<DIR>(v[r], w[(r - 1) * nt + t]);
+    rf::dft<DIR, E>(v);
   }
 }
 
