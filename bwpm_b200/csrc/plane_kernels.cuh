@@ -73,9 +73,9 @@ constexpr int table_blocks() {
 // followed by their lo blocks), pair index (into the step's pair-id plane), reflection flag. The
 // records of every step live in device memory (a per-solve pool built once), so a kernel reads
 // pass j as one uniform load instead of indexing a by-value parameter array.
-// `scalar`: a complex64 transmission between equal indices in 3D, whose operator is the
-// propagator e^{i k_z dz} times the identity (T = 1 for ñ_r = ñ_s): its table holds only that
-// value (hi block, then lo block: 2·N entries) and both components are multiplied by it.
+// `scalar`: a transmission between equal indices in 3D, whose operator is the propagator
+// e^{i k_z dz} times the identity (T = 1 for ñ_r = ñ_s): its table holds only that value
+// (complex64: hi block, then lo block) and both components are multiplied by it.
 struct PassRec {
   const void* tab;
   int pair;
@@ -619,23 +619,42 @@ __global__ void k_convert(cx<To>* dst, const cx<From>* src, long long count) {
 }
 
 // Operator table of one (kind, ñ_r, ñ_s): entry q is mode (x, y) = (q mod nx, q div nx), or with
-// `transposed` (3D solves, read column by column) (q div ny, q mod ny).
-// `scalar` (complex64, equal indices): only m00 = e^{i k_z dz}/N, hi block then lo block.
+// `transposed` (3D solves, read column by column) (q div ny, q mod ny), with `quarter` of the modes
+// x ≤ nx/2, y ≤ ny/2 only (plane_rf.cuh).
+// `scalar` (equal indices): only m00 = e^{i k_z dz}. Complex64 entries are over N, as hi and lo:
+// blocks of each, or with `quarter` side by side.
 template <typename T>
 __global__ void k_build_table(cx<T>* out, int kind, cd nr, cd ns, int ny, int nx, double dy,
-                              double dx, double k0, double dz, int transposed, int scalar) {
-  const long long n = static_cast<long long>(ny) * nx;
+                              double dx, double k0, double dz, int transposed, int scalar,
+                              int quarter) {
+  const int ty = quarter ? ny / 2 + 1 : ny, tx = quarter ? nx / 2 + 1 : nx;
+  const long long n = static_cast<long long>(ty) * tx;
   const long long q = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   if (q >= n) return;
-  const long long xi = transposed ? q / ny : q % nx;
-  const long long yi = transposed ? q % ny : q / nx;
+  const double points = static_cast<double>(static_cast<long long>(ny) * nx);
+  const long long xi = transposed ? q / ty : q % tx;
+  const long long yi = transposed ? q % ty : q / tx;
   const double kx = fftfreq(xi, nx, dx);
   const double ky = fftfreq(yi, ny, dy);
   cd m[3];
   operator_matrix(kind, kx, ky, nr, ns, k0, dz, m);
-  if constexpr (sizeof(T) != sizeof(double)) {
+  if constexpr (sizeof(T) == sizeof(double)) {
     if (scalar) {
-      const cd v = m[0] / static_cast<double>(n);
+      out[q] = m[0];
+      return;
+    }
+  } else {
+    if (quarter) {  // hi and lo side by side: one 16-byte load per entry
+      for (int e = 0; e < (scalar ? 1 : 3); ++e) {
+        const cd v = m[e] / points;
+        const cf hi = cast<float>(v);
+        out[2 * (e * n + q)] = hi;
+        out[2 * (e * n + q) + 1] = cf{static_cast<float>(v.re - hi.re), static_cast<float>(v.im - hi.im)};
+      }
+      return;
+    }
+    if (scalar) {
+      const cd v = m[0] / points;
       const cf hi = cast<float>(v);
       out[q] = hi;
       out[n + q] = cf{static_cast<float>(v.re - hi.re), static_cast<float>(v.im - hi.im)};
@@ -646,7 +665,7 @@ __global__ void k_build_table(cx<T>* out, int kind, cd nr, cd ns, int ny, int nx
     if constexpr (sizeof(T) == sizeof(double)) {
       out[e * n + q] = m[e];
     } else {  // FP32 fields: M/N as hi + lo (the inverse transform's 1/N folded in)
-      const cd v = m[e] / static_cast<double>(n);
+      const cd v = m[e] / points;
       const cf hi = cast<float>(v);
       out[e * n + q] = hi;
       out[(3 + e) * n + q] = cf{static_cast<float>(v.re - hi.re), static_cast<float>(v.im - hi.im)};

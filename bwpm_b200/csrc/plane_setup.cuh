@@ -113,6 +113,19 @@ __global__ void __launch_bounds__(kSetupThreads)
   if (rowoff && threadIdx.x == 0) rowoff[rows] = running;
 }
 
+// One warp per row of the pair-id planes: bit i of row_pairs[row] when pair i occurs in it (a step
+// has at most kMaxPasses/2 = 64 pairs).
+__global__ void k_setup_row_pairs(const std::uint8_t* pid, long long rows, int nx,
+                                  unsigned long long* row_pairs) {
+  const long long row = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
+  if (row >= rows) return;
+  const int lane = threadIdx.x & 31;
+  unsigned long long m = 0;
+  for (int x = lane; x < nx; x += 32) m |= 1ull << pid[row * nx + x];
+  for (int o = 16; o > 0; o >>= 1) m |= __shfl_xor_sync(0xffffffffu, m, o);
+  if (lane == 0) row_pairs[row] = m;
+}
+
 // int32 labels → uint8 (device); sets *bad when a label is outside [0, m).
 __global__ void k_labels_to_u8(const std::int32_t* in, std::uint8_t* out, long long count, int m,
                                int* bad) {

@@ -100,6 +100,9 @@ class PlaneSolver final : public Solver {
   LaunchShape step_rows_shape() const;
   std::size_t n() const { return in_.ny * in_.nx; }
   bool is2d() const { return in_.nx == 1; }
+  // 3D transmissions between equal indices keep one value per mode (the general kernels: in
+  // complex64 only)
+  bool scalar_tables() const { return !is2d() && (rf_y_.cols || sizeof(T) != sizeof(double)); }
   cd index_of(int label) const {
     return label < 0 ? in_.index_before : in_.indices[static_cast<std::size_t>(label)];
   }
@@ -111,6 +114,28 @@ class PlaneSolver final : public Solver {
   void launch(K kernel, dim3 grid, dim3 block, std::size_t smem, A... args) {
     kernel<<<grid, block, smem, stream_>>>(args...);
     check_cuda(cudaGetLastError(), "kernel launch");
+    ++launches_;
+  }
+
+  // a register-resident 3D kernel, its prologue overlapping the end of the kernel before
+  // (programmatic dependent launch)
+  template <class A>
+  void launch_rf(const void* fn, const RfKernels& k, unsigned grid, A a, const PassRec* ps, int npass,
+                 const FftPlan& plan) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(k.threads);
+    cfg.dynamicSmemBytes = fn == k.cols ? k.cols_smem : k.rows_smem;
+    cfg.stream = stream_;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int lines = k.lines;
+    FftPlan p = plan;
+    void* args[] = {&a, &ps, &npass, &p, &lines};
+    check_cuda(cudaLaunchKernelExC(&cfg, fn, args), "3D step kernel");
     ++launches_;
   }
 
@@ -155,9 +180,12 @@ class PlaneSolver final : public Solver {
   int sms_ = 148;
   LaunchShape rows2_, rows3_, sel_, cols1_, cols2_, cols3_;
   std::int64_t launches_ = 0, gmres_applies_ = 0;
-  // complex64 3D: the fixed-length step kernels (plane_rf.cuh) when both lateral sizes have one
+  // 3D: the register-resident step kernels (plane_rf.cuh) when both lateral sizes have them; the
+  // operator tables then hold a quarter plane
   RfKernels rf_y_, rf_x_;
-  DevBuf<Tw<float>> tw_rf_y_, tw_rf_x_;
+  HostPlan rf_plan_y_, rf_plan_x_;
+  DevBuf<Tw<T>> tw_rf_y_, tw_rf_x_;
+  DevBuf<unsigned long long> row_pairs_;  // per pair-id plane and row: the pairs that occur
   bool cols_bulk_ = false;  // 3D column kernel with bulk copies (k_cols_step_bulk)
   int cols_bulk_threads_ = 256, cols_bulk_group_ = 1;
   DevBuf<int> status_;      // set by a kernel whose bounded wait gave up
@@ -528,27 +556,29 @@ void PlaneSolver<T>::setup() {
                    (const void*)k_rows_select<T>,
                    (const void*)k_cols_fft<-1, T>, (const void*)k_cols_fft<1, T>})
       check_cuda(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024), "smem");
-    // complex64: fixed-length kernels where ny and nx have them (whole CTAs of lines);
-    // BWPM_3D_KERNELS=general selects the general kernels
+    // register-resident kernels where ny and nx have them; BWPM_3D_KERNELS=general selects the
+    // general kernels
     const char* kk = std::getenv("BWPM_3D_KERNELS");
-    if (sizeof(T) == sizeof(float) && !(kk && std::strcmp(kk, "general") == 0)) {
-      RfKernels ky = rf_kernels(nyi), kx = rf_kernels(static_cast<int>(in_.nx));
-      if (ky.cols && kx.rows && in_.nx % ky.lines == 0 && in_.ny % kx.lines == 0) {
+    if (!(kk && std::strcmp(kk, "general") == 0)) {
+      RfKernels ky = rf_kernels<T>(nyi), kx = rf_kernels<T>(static_cast<int>(in_.nx));
+      if (ky.cols && kx.rows) {
         rf_y_ = ky;
         rf_x_ = kx;
-        auto upload_rf = [&](const RfKernels& k, int len, DevBuf<Tw<float>>& d) {
-          const std::vector<Tw<float>> t = twiddles_for<float>(make_plan_radices(len, k.radices));
-          d.alloc(t.size(), stream_);
-          d.upload(t.data(), t.size());
-        };
-        upload_rf(rf_y_, nyi, tw_rf_y_);
-        upload_rf(rf_x_, static_cast<int>(in_.nx), tw_rf_x_);
-        check_cuda(cudaFuncSetAttribute((const void*)rf_y_.cols,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(rf_y_.smem)), "smem");
-        check_cuda(cudaFuncSetAttribute((const void*)rf_x_.rows,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(rf_x_.smem)), "smem");
+        rf_plan_y_ = make_plan_radices(nyi, ky.radices);
+        rf_plan_x_ = make_plan_radices(static_cast<int>(in_.nx), kx.radices);
+        upload_tw(rf_plan_y_, tw_rf_y_);
+        upload_tw(rf_plan_x_, tw_rf_x_);
+        check_cuda(cudaFuncSetAttribute(rf_y_.cols, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        static_cast<int>(rf_y_.cols_smem)), "smem");
+        check_cuda(cudaFuncSetAttribute(rf_x_.rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        static_cast<int>(rf_x_.rows_smem)), "smem");
+        if (pid_pool_.n) {  // whole pair-id planes
+          const std::size_t rows = pid_pool_.n / in_.nx;
+          row_pairs_.alloc(rows, stream_);
+          launch(k_setup_row_pairs, dim3(ceil_div(rows, std::size_t{8})), dim3(256), 0,
+                 (const std::uint8_t*)pid_pool_.ptr, static_cast<long long>(rows),
+                 static_cast<int>(in_.nx), row_pairs_.ptr);
+        }
       }
     }
   }
@@ -557,7 +587,7 @@ void PlaneSolver<T>::setup() {
     for (auto& pr : steps_[p].pairs) {
       const cd nr = index_of(pr.first), ns = index_of(pr.second);
       const bool same = nr.re == ns.re && nr.im == ns.im;
-      table(kFwdT, nr, ns, sizeof(T) != sizeof(double) && !is2d() && same);
+      table(kFwdT, nr, ns, scalar_tables() && same);
     }
   // Born: potential V = 2ñ₀k₀²δn per host slab, full-plane source stores
   if (!hosts_.empty()) {
@@ -697,10 +727,12 @@ const cx<T>* PlaneSolver<T>::table(int kind, cd nr, cd ns, bool scalar) {
   auto key = std::make_tuple(kind + (scalar ? 8 : 0), nr.re, nr.im, ns.re, ns.im);
   auto it = tables_.find(key);
   if (it != tables_.end()) return it->second.ptr;
-  DevBuf<C> t((scalar ? 2 : table_blocks<T>()) * n(), stream_);
-  launch(k_build_table<T>, dim3(ceil_div(n(), kThreads)), dim3(kThreads), 0, t.ptr, kind, nr, ns,
+  const int quarter = rf_y_.cols ? 1 : 0;
+  const std::size_t pts = quarter ? (in_.ny / 2 + 1) * (in_.nx / 2 + 1) : n();
+  DevBuf<C> t((scalar ? (sizeof(T) == sizeof(double) ? 1 : 2) : table_blocks<T>()) * pts, stream_);
+  launch(k_build_table<T>, dim3(ceil_div(pts, kThreads)), dim3(kThreads), 0, t.ptr, kind, nr, ns,
          static_cast<int>(in_.ny), static_cast<int>(in_.nx), in_.dy, in_.dx, in_.k0, in_.dz,
-         is2d() ? 0 : 1, scalar ? 1 : 0);
+         is2d() ? 0 : 1, scalar ? 1 : 0, quarter);
   const C* ptr = t.ptr;
   tables_.emplace(key, std::move(t));
   return ptr;
@@ -734,8 +766,8 @@ void PlaneSolver<T>::ensure_passes(bool with_backward) {
           const bool same = nr.re == ns.re && nr.im == ns.im;
           if (pass == 1 && same) continue;
           const int kind = pass == 0 ? (backward ? kBwdT : kFwdT) : (backward ? kBwdR : kFwdR);
-          // complex64 3D transmissions between equal indices: T = 1, the propagator alone
-          const bool scalar = sizeof(T) != sizeof(double) && !is2d() && pass == 0 && same;
+          // 3D transmissions between equal indices: T = 1, the propagator alone
+          const bool scalar = scalar_tables() && pass == 0 && same;
           host.push_back(PassRec{table(kind, nr, ns, scalar), static_cast<int>(i), pass,
                                  scalar ? 1 : 0});
           ++(pass == 0 ? pass_nt_[d][s] : pass_nr_[d][s]);
@@ -832,32 +864,29 @@ void PlaneSolver<T>::step(int s, bool backward, bool reflect, const C* in, C* ou
   if (!x_ready)  // the x transform of the step's input, stored transposed for the column kernel
     launch(k_rows_fft<-1, T, true>, dim3(ceil_div(ny, sel_.rows)), dim3(sel_.threads), sel_.smem, in,
            xbuf_.ptr, ny, nx, 2, sel_.rows, hx_.plan, tw_x_.ptr);
-  if constexpr (sizeof(T) == sizeof(float)) {
-    if (rf_y_.cols) {
-      ColStep<float> c{xbuf_.ptr, work_.ptr, want_spec ? spec_.ptr : nullptr, ny, nx, 0,
-                       status_.ptr};
-      launch(rf_y_.cols, dim3(nx / rf_y_.lines), dim3(kRfThreads), rf_y_.smem, c, ps, npass,
-             (const Tw<float>*)tw_rf_y_.ptr);
-      RowSelect<float> r;
-      r.work = work_.ptr;
-      r.out = out;
-      r.pid = pid;
-      r.mask = mask_.ptr;
-      r.iface = iface;
-      r.rowoff = st.rowoff_off >= 0 ? rowoff_pool_.ptr + st.rowoff_off : nullptr;
-      r.refl_out = refl_out;
-      r.add = add;
-      r.xnext = x_next ? xbuf_.ptr : nullptr;
-      r.ny = ny;
-      r.nx = nx;
-      r.rows = rf_x_.lines;
-      r.group = 1;
-      r.store_out = need_out ? 1 : 0;
-      r.inv_n = inv_n;
-      launch(rf_x_.rows, dim3(ny / rf_x_.lines), dim3(kRfThreads), rf_x_.smem, r, ps, npass,
-             (const Tw<float>*)tw_rf_x_.ptr);
-      return;
-    }
+  if (rf_y_.cols) {
+    const unsigned long long* pairs = pid ? row_pairs_.ptr + st.pid_off / in_.nx : nullptr;
+    RfCols<T> c{xbuf_.ptr, work_.ptr, want_spec ? spec_.ptr : nullptr, pairs, tw_rf_y_.ptr, ny, nx,
+                status_.ptr};
+    launch_rf(rf_y_.cols, rf_y_, rf_column_ctas(nx, rf_y_.lines), c, ps, npass, rf_plan_y_.plan);
+    RfRows<T> r;
+    r.work = work_.ptr;
+    r.out = out;
+    r.pid = pid;
+    r.row_pairs = pairs;
+    r.mask = mask_.ptr;
+    r.iface = iface;
+    r.rowoff = st.rowoff_off >= 0 ? rowoff_pool_.ptr + st.rowoff_off : nullptr;
+    r.refl_out = refl_out;
+    r.add = add;
+    r.xnext = x_next ? xbuf_.ptr : nullptr;
+    r.tw = tw_rf_x_.ptr;
+    r.ny = ny;
+    r.nx = nx;
+    r.store_out = need_out ? 1 : 0;
+    r.inv_n = inv_n;
+    launch_rf(rf_x_.rows, rf_x_, ceil_div(ny, rf_x_.lines), r, ps, npass, rf_plan_x_.plan);
+    return;
   }
   if (cols_bulk_) {
     ColStep<T> c{xbuf_.ptr, work_.ptr, want_spec ? spec_.ptr : nullptr, ny, nx, cols_bulk_group_,
