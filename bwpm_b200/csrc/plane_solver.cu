@@ -14,6 +14,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <set>
 #include <string>
 #include <tuple>
@@ -87,9 +88,11 @@ class PlaneSolver final : public Solver {
   void arnoldi_step(int j, bool in_graph, double tol_bnorm);
   void gmres_alloc();
   void build_born_graph();
-  // the forward/backward sweeps of a run (device work only, unless Born slabs need GMRES)
+  // the forward/backward sweeps of a run (device work only, unless Born slabs need GMRES);
+  // swept(k) is called when sweep k (forward 2·it, backward 2·it + 1) has been enqueued
+  template <typename F>
   void sweeps(int iterations, const std::vector<int>& keep_slot, DevBuf<C>& kept_f, DevBuf<C>& kept_b,
-              DevBuf<C>& t_iter, DevBuf<C>& r_iter);
+              DevBuf<C>& t_iter, DevBuf<C>& r_iter, F swept);
   // the sweeps of a 2D run without Born slabs, as one launch (chain2d.cuh)
   void chain(int iterations, const std::vector<int>& keep_slot, bool any_keep, DevBuf<C>& kept_f,
              DevBuf<C>& kept_b, DevBuf<C>& t_iter, DevBuf<C>& r_iter);
@@ -141,6 +144,8 @@ class PlaneSolver final : public Solver {
 
   SolverInput in_;
   OwnedStream stream_;  // first: outlives the stream-ordered buffers below
+  OwnedStream copy_stream_;                               // 3D: downloads of earlier sweeps' planes
+  std::vector<std::unique_ptr<OwnedEvent>> sweep_done_;   // per sweep of a run
   HostPlan hy_, hx_;
   DevBuf<Tw<T>> tw_y_, tw_x_;
   std::vector<StepInfo> steps_;
@@ -1270,8 +1275,9 @@ void PlaneSolver<T>::born_emission(int slot, int dir, C* plane) {
 }
 
 template <typename T>
+template <typename F>
 void PlaneSolver<T>::sweeps(int iterations, const std::vector<int>& keep_slot, DevBuf<C>& kept_f,
-                            DevBuf<C>& kept_b, DevBuf<C>& t_iter, DevBuf<C>& r_iter) {
+                            DevBuf<C>& kept_b, DevBuf<C>& t_iter, DevBuf<C>& r_iter, F swept) {
   const std::size_t nn = n();
   const long long n2 = 2 * static_cast<long long>(nn);
   const int nz = static_cast<int>(in_.nz);
@@ -1309,8 +1315,9 @@ void PlaneSolver<T>::sweeps(int iterations, const std::vector<int>& keep_slot, D
       if (it > 0 && host) add_plane_scaled(e, born_fwd_.ptr + st.host_slot * n2, nullptr);  // born_fwd[p + 1]
       if (last && keep_slot[p + 1] >= 0) copy(kept_f.ptr + keep_slot[p + 1] * n2, e);
     }
-    if (iterations > 0) copy(t_iter.ptr + it * n2, e);
     if (iterations == 0) break;
+    copy(t_iter.ptr + it * n2, e);
+    swept(2 * it);
     check_cuda(cudaMemsetAsync(e, 0, n2 * sizeof(C), stream_), "memset");
     if (born && steps_[nz - 1].host_slot >= 0)
       add_plane_scaled(e, born_bwd_.ptr + steps_[nz - 1].host_slot * n2, nullptr);  // born_bwd[nz]
@@ -1335,6 +1342,7 @@ void PlaneSolver<T>::sweeps(int iterations, const std::vector<int>& keep_slot, D
       if (last && keep_slot[p - 1] >= 0) copy(kept_b.ptr + keep_slot[p - 1] * n2, e);
     }
     copy(r_iter.ptr + it * n2, e);
+    swept(2 * it + 1);
   }
   last_e_ = e;
 }
@@ -1360,32 +1368,72 @@ void PlaneSolver<T>::run(const cd* field, int iterations, const std::int64_t* ke
   check_cuda(cudaMemcpyAsync(stage_.ptr, field, n2 * sizeof(cd), cudaMemcpyHostToDevice, stream_), "field upload");
   launch(k_convert<T, double>, dim3(ceil_div(n2, kThreads)), dim3(kThreads), 0, input_.ptr,
          (const cd*)stage_.ptr, n2);
-  if (chain_.fn)
-    chain(iterations, keep_slot, nkeep > 0, kept_f, kept_b, t_iter, r_iter);
-  else
-    sweeps(iterations, keep_slot, kept_f, kept_b, t_iter, r_iter);
-  C* e = last_e_;
-  // outputs
-  auto download = [&](const C* src, cd* dst) {
+  // FP64 planes are downloaded as they are, complex64 ones through a conversion
+  auto download = [&](const C* src, cd* dst, cudaStream_t s) {
     if (!dst) return;
-    launch(k_convert<double, T>, dim3(ceil_div(n2, kThreads)), dim3(kThreads), 0, stage_.ptr, src, n2);
-    check_cuda(cudaMemcpyAsync(dst, stage_.ptr, n2 * sizeof(cd), cudaMemcpyDeviceToHost, stream_), "download");
-    check_cuda(cudaStreamSynchronize(stream_), "download");
+    const cd* from = reinterpret_cast<const cd*>(src);
+    if constexpr (sizeof(T) != sizeof(double)) {
+      k_convert<double, T><<<ceil_div(n2, kThreads), kThreads, 0, s>>>(stage_.ptr, src, n2);
+      check_cuda(cudaGetLastError(), "kernel launch");
+      ++launches_;
+      from = stage_.ptr;
+    }
+    check_cuda(cudaMemcpyAsync(dst, from, n2 * sizeof(cd), cudaMemcpyDeviceToHost, s), "download");
+    check_cuda(cudaStreamSynchronize(s), "download");
   };
-  download(iterations > 0 ? t_iter.ptr + (iterations - 1) * n2 : e, out.transmitted);
-  if (out.reflected) {
-    if (iterations > 0)
-      download(r_iter.ptr + (iterations - 1) * n2, out.reflected);
-    else
-      std::memset(static_cast<void*>(out.reflected), 0, n2 * sizeof(cd));
+  // the plane of sweep k: its iteration's output and, in the last iteration, the run's
+  auto download_sweep = [&](int k, cudaStream_t s) {
+    const int it = k / 2;
+    const C* src = (k % 2 ? r_iter.ptr : t_iter.ptr) + it * n2;
+    cd* each = k % 2 ? out.reflected_iter : out.transmitted_iter;
+    cd* last = it == iterations - 1 ? (k % 2 ? out.reflected : out.transmitted) : nullptr;
+    download(src, each ? each + it * n2 : nullptr, s);
+    download(src, last, s);
+  };
+  int downloaded = 0;  // sweeps whose planes are on the host
+  if (chain_.fn) {
+    chain(iterations, keep_slot, nkeep > 0, kept_f, kept_b, t_iter, r_iter);
+  } else {
+    // a sweep's plane goes to the host on its own stream while the next sweep, already
+    // enqueued, runs
+    const bool overlap = iterations > 0 && !is2d();
+    if (overlap) {
+      if (!copy_stream_.s) copy_stream_.create();
+      while (sweep_done_.size() < static_cast<std::size_t>(2 * iterations)) {
+        sweep_done_.emplace_back(std::make_unique<OwnedEvent>());
+        sweep_done_.back()->create();
+      }
+    }
+    try {
+      sweeps(iterations, keep_slot, kept_f, kept_b, t_iter, r_iter, [&](int k) {
+        if (!overlap) return;
+        check_cuda(cudaEventRecord(*sweep_done_[k], stream_), "event");
+        if (k == 0) return;
+        check_cuda(cudaStreamWaitEvent(copy_stream_, *sweep_done_[k - 1], 0), "wait");
+        download_sweep(k - 1, copy_stream_);
+        downloaded = k;
+      });
+    } catch (...) {  // the buffers of this call outlive the copies in flight
+      if (copy_stream_.s) cudaStreamSynchronize(copy_stream_);
+      throw;
+    }
   }
-  for (int it = 0; it < iterations; ++it) {
-    if (out.transmitted_iter) download(t_iter.ptr + it * n2, out.transmitted_iter + it * n2);
-    if (out.reflected_iter) download(r_iter.ptr + it * n2, out.reflected_iter + it * n2);
+  // the remaining outputs; while the last sweep still runs, their pages are brought in (the
+  // caller's arrays are new: the first write of each page faults)
+  if (iterations > 0) {
+    if (downloaded > 0)
+      for (cd* p : {out.reflected_iter ? out.reflected_iter + (iterations - 1) * n2 : nullptr, out.reflected})
+        if (p)
+          for (long long i = 0; i < n2; i += 4096 / static_cast<long long>(sizeof(cd)))
+            const_cast<volatile cd*>(p)[i].re = 0.0;
+    for (int k = downloaded; k < 2 * iterations; ++k) download_sweep(k, stream_);
+  } else {
+    download(last_e_, out.transmitted, stream_);
+    if (out.reflected) std::memset(static_cast<void*>(out.reflected), 0, n2 * sizeof(cd));
   }
   for (std::size_t i = 0; i < nkeep; ++i) {
-    if (out.forward) download(kept_f.ptr + i * n2, out.forward + i * n2);
-    if (out.backward && iterations > 0) download(kept_b.ptr + i * n2, out.backward + i * n2);
+    if (out.forward) download(kept_f.ptr + i * n2, out.forward + i * n2, stream_);
+    if (out.backward && iterations > 0) download(kept_b.ptr + i * n2, out.backward + i * n2, stream_);
   }
   out.stored_values = iterations > 0 ? 2 * iface_total_ : 0;
   check_cuda(cudaStreamSynchronize(stream_), "synchronize");
