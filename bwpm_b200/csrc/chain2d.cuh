@@ -63,9 +63,11 @@ struct FixedLine {
   cx<T>*b0, *b1;
   const Tw<T>* tw;
   int t, phase;
-  __device__ __forceinline__ FixedLine(const FftPlan&, const unsigned*, int, const Tw<T>* w, cx<T>* base)
-      : b0(base), b1(base + rf::padded<T>(N)), tw(w), t(threadIdx.x), phase(0) {}
+  __device__ __forceinline__ FixedLine(const FftPlan&, const unsigned*, int, const Tw<T>* w, cx<T>* base,
+                                       int thread, int)
+      : b0(base), b1(base + rf::padded<T>(N)), tw(w), t(thread), phase(0) {}
   __device__ __forceinline__ int n() const { return N; }
+  __device__ __forceinline__ int threads() const { return NT_; }
   __device__ __forceinline__ int pos(int m) const { return t + m * NT_; }
   __device__ __forceinline__ bool own() const { return true; }
   template <int DIR>
@@ -85,17 +87,19 @@ struct RuntimeLine {
   const unsigned* magic;
   cx<T>*b0, *b1;
   const Tw<T>* tw;
-  int t, nt, n_, phase;
+  int t, gn, nt, n_, phase;
+  // thread `thread` of the line's `group` threads
   __device__ __forceinline__ RuntimeLine(const FftPlan& p, const unsigned* mg, int len, const Tw<T>* w,
-                                         cx<T>* base)
-      : plan(p), magic(mg), b0(base), b1(base + rf::padded<T>(len)), tw(w), t(threadIdx.x), nt(len / E_),
-        n_(len), phase(0) {}
+                                         cx<T>* base, int thread, int group)
+      : plan(p), magic(mg), b0(base), b1(base + rf::padded<T>(len)), tw(w), t(thread), gn(group),
+        nt(len / E_), n_(len), phase(0) {}
   __device__ __forceinline__ int n() const { return n_; }
+  __device__ __forceinline__ int threads() const { return nt; }
   __device__ __forceinline__ int pos(int m) const { return t + m * nt; }
   __device__ __forceinline__ bool own() const { return t < nt; }
   template <int DIR>
   __device__ __forceinline__ void fft(cx<T> (&v)[E]) {
-    rg::gfft<DIR, E>(v, b0, b1, phase, plan, magic, tw, t, nt);
+    rg::gfft<DIR, E>(v, b0, b1, phase, plan, magic, tw, t, nt, gn);
   }
 };
 
@@ -145,7 +149,7 @@ __global__ void __launch_bounds__(Line::kMaxThreads, 1)
     __syncthreads();
   }
   C* lines = reinterpret_cast<C*>(smem_raw);
-  Line ln(s_plan, s_magic, a.n, a.tw, lines);
+  Line ln(s_plan, s_magic, a.n, a.tw, lines, t, nthr);
   const int n = ln.n(), pn = rf::padded<T>(n);
   const bool own = ln.own();
   // beside the two exchange lines, where they fit: the stage twiddles, the mask (8 bytes a point

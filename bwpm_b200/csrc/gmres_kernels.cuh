@@ -104,7 +104,7 @@ __global__ void k_norm_scale(cx<T>* out, const cx<T>* in, const cd* dot, double*
 }
 
 // g = (β, 0, …, 0) with β = √Re(dot); the cycle's flags cleared; tolb = tol·‖rhs‖.
-__global__ void k_gmres_start(GmresState* s, double tol_bnorm) {
+static __global__ void k_gmres_start(GmresState* s, double tol_bnorm) {
   const int i = threadIdx.x;
   if (i <= kGmresRestart) s->g[i] = cd{i == 0 ? sqrt(s->dot.re) : 0.0, 0.0};
   if (i < kGmresRestart) s->flag[i] = 0;
@@ -138,7 +138,7 @@ __device__ __forceinline__ void gmres_givens(GmresState* s, int j, double tol_bn
   s->flag[j] = (hypot(s->g[j + 1].re, s->g[j + 1].im) <= tol_bnorm || hnext == 0.0) ? 1 : 0;
 }
 
-__global__ void k_gmres_givens(GmresState* s, int j, double tol_bnorm) {
+static __global__ void k_gmres_givens(GmresState* s, int j, double tol_bnorm) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   gmres_givens(s, j, tol_bnorm);
 }
@@ -146,7 +146,7 @@ __global__ void k_gmres_givens(GmresState* s, int j, double tol_bnorm) {
 // The same as the last node of Arnoldi step j in the cycle graph: the tolerance comes from the
 // state, and the condition of step j + 1's node (`next`, when there is one) is set unless step j
 // has converged.
-__global__ void k_gmres_givens_cond(GmresState* s, int j, GmresConds c) {
+static __global__ void k_gmres_givens_cond(GmresState* s, int j, GmresConds c) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   gmres_givens(s, j, s->tolb);
   if (j + 1 < kGmresRestart) cudaGraphSetConditional(c.step[j + 1], s->flag[j] ? 0u : 1u);
@@ -154,7 +154,7 @@ __global__ void k_gmres_givens_cond(GmresState* s, int j, GmresConds c) {
 
 // Back substitution for the first `used` unknowns (cpp/src/solver.cpp:193-199); used < 0: the
 // count the Born-step graph left in the state.
-__global__ void k_gmres_backsolve(GmresState* s, int used) {
+static __global__ void k_gmres_backsolve(GmresState* s, int used) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   if (used < 0) used = s->used;
   constexpr int m = kGmresRestart;
@@ -170,7 +170,7 @@ __global__ void k_gmres_backsolve(GmresState* s, int used) {
 // is the host loop's, in the same FP64 operations.
 
 // After ‖rhs‖²: ‖rhs‖ = 0 ends the solve at once (y = rhs = 0), else the restarts begin.
-__global__ void k_gmres_init(GmresState* s, double tol, GmresConds c) {
+static __global__ void k_gmres_init(GmresState* s, double tol, GmresConds c) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   const double bnorm = sqrt(s->dot.re);
   s->tolb = tol * bnorm;
@@ -180,7 +180,7 @@ __global__ void k_gmres_init(GmresState* s, double tol, GmresConds c) {
 
 // After β² = ‖rhs − A·y‖²: β ≤ tol·‖rhs‖ ends the solve; else a cycle runs, unless the solve
 // has used its 100 restarts (then `err`).
-__global__ void k_gmres_restart(GmresState* s, GmresConds c) {
+static __global__ void k_gmres_restart(GmresState* s, GmresConds c) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   s->applies += 1;
   const double beta = sqrt(s->dot.re);
@@ -198,13 +198,13 @@ __global__ void k_gmres_restart(GmresState* s, GmresConds c) {
 }
 
 // Before a cycle: step 0 runs, the others wait for their predecessor.
-__global__ void k_gmres_arm(GmresConds c) {
+static __global__ void k_gmres_arm(GmresConds c) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   for (int j = 0; j < kGmresRestart; ++j) cudaGraphSetConditional(c.step[j], j == 0 ? 1u : 0u);
 }
 
 // After a cycle: used = steps up to the first converged one (all if none); `done` when one did.
-__global__ void k_gmres_cycle_done(GmresState* s, GmresConds c) {
+static __global__ void k_gmres_cycle_done(GmresState* s, GmresConds c) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   int used = kGmresRestart;
   unsigned done = 0u;
@@ -220,7 +220,7 @@ __global__ void k_gmres_cycle_done(GmresState* s, GmresConds c) {
 }
 
 // After ‖rhs − A·y‖² of a converged cycle: within 10·tol·‖rhs‖ ends the solve, else restart.
-__global__ void k_gmres_final(GmresState* s, GmresConds c) {
+static __global__ void k_gmres_final(GmresState* s, GmresConds c) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   s->applies += 1;
   if (sqrt(s->dot.re) <= s->tolb * 10.0) cudaGraphSetConditional(c.active, 0u);

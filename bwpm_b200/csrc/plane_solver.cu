@@ -20,6 +20,7 @@
 #include <tuple>
 #include <unordered_map>
 
+#include "born2d.cuh"
 #include "born_kernels.cuh"
 #include "chain2d.cuh"
 #include "devbuf.hpp"
@@ -88,6 +89,9 @@ class PlaneSolver final : public Solver {
   void arnoldi_step(int j, bool in_graph, double tol_bnorm);
   void gmres_alloc();
   void build_born_graph();
+  // a whole Born slab in one launch (born2d.cuh); step_tab/in/out as in BornSlab
+  void born_slab(int slot, int dir, const C* in, const C* step_tab, C* out, const C* incoming,
+                 C* radiated, const T* mask);
   // the forward/backward sweeps of a run (device work only, unless Born slabs need GMRES);
   // swept(k) is called when sweep k (forward 2·it, backward 2·it + 1) has been enqueued
   template <typename F>
@@ -177,6 +181,12 @@ class PlaneSolver final : public Solver {
   // launch shapes
   int thr2d_ = 32, thr_line3_ = 32;
   bool line_ept8_ = false;  // 2D line transforms with 8 values per thread (k_line_fft)
+  // 2D Born slabs: one cluster launch per slab (fn null: the kernels and graphs above)
+  BornKernel born_k_;
+  HostPlan born_plan_;
+  DevBuf<Tw<T>> tw_born_;
+  std::map<std::pair<double, double>, DevBuf<cd>> born_modes_;  // per distinct host index
+  DevBuf<C> born_basis_;
   // 2D without Born slabs: one launch runs all sweeps (fn null: a launch per step instead)
   ChainKernel chain_;
   HostPlan chain_plan_;
@@ -612,6 +622,38 @@ void PlaneSolver<T>::setup() {
     t3_.alloc(3 * nn, stream_);
     sources_.alloc(6 * nn, stream_);
     for (auto* b : {&g_x_, &g_rhs_, &g_y_, &g_w_, &g_tmp_, &inc_}) b->alloc(2 * nn, stream_);
+    // BWPM_GMRES=graph|host selects the multi-kernel forms
+    if (is2d() && !std::getenv("BWPM_GMRES")) born_k_ = born_kernel<T>(static_cast<int>(in_.ny));
+    if (born_k_.fn) {
+      const int m = static_cast<int>(in_.ny) / born_k_.ctas;
+      born_plan_ = make_plan_radices(m, born_k_.radices);
+      HostPlan all = born_plan_;  // stage twiddles, then w_N^{c·k}
+      all.twiddles.resize(static_cast<std::size_t>(m - 1));
+      if (born_k_.ctas > 1)
+        for (int c = 0; c < born_k_.ctas; ++c)
+          for (int k = 0; k < m; ++k) {
+            const double ang = -6.283185307179586476925286766559 *
+                               static_cast<double>((static_cast<long long>(c) * k) % static_cast<long long>(in_.ny)) /
+                               static_cast<double>(in_.ny);
+            all.twiddles.push_back(cd{std::cos(ang), std::sin(ang)});
+          }
+      if (all.twiddles.empty()) all.twiddles.push_back(cd{1.0, 0.0});
+      upload_tw(all, tw_born_);
+      for (std::size_t i = 0; i < hosts_.size(); ++i) {
+        DevBuf<cd>& d = born_modes_[{hosts_[i].re, hosts_[i].im}];
+        if (d.n) continue;
+        d.alloc(kBtCount * nn, stream_);
+        launch(k_born_modes, dim3(ceil_div(nn, kThreads)), dim3(kThreads), 0, d.ptr, born_grid(static_cast<int>(i)));
+      }
+      const int mb = (m + born_k_.ctas - 1) / born_k_.ctas;
+      born_basis_.alloc(static_cast<std::size_t>(born_k_.ctas) * kBornVectors * 2 * born_k_.ctas * mb, stream_);
+      gst_.alloc(1, stream_);
+      check_cuda(cudaMemsetAsync(gst_.ptr, 0, sizeof(GmresState), stream_), "memset");
+      status_.alloc(1, stream_);
+      check_cuda(cudaMemsetAsync(status_.ptr, 0, sizeof(int), stream_), "memset");
+      check_cuda(cudaFuncSetAttribute(born_k_.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(born_k_.smem)), "smem");
+    }
   }
   check_cuda(cudaStreamSynchronize(stream_), "setup");  // this solver's stream only
 }
@@ -1246,6 +1288,44 @@ void PlaneSolver<T>::born_step(const C* spec, C* inc, int slot, int dir) {
   fft_plane(g_y_.ptr, inc, 2, +1);
 }
 
+template <typename T>
+void PlaneSolver<T>::born_slab(int slot, int dir, const C* in, const C* step_tab, C* out,
+                               const C* incoming, C* radiated, const T* mask) {
+  BornSlab<T> a;
+  a.in = in;
+  a.spec = spec_.ptr;
+  a.step_tab = step_tab;
+  a.out = out;
+  a.incoming = incoming;
+  a.radiated = radiated;
+  a.mask = mask;
+  a.pot = pot_.ptr + static_cast<long long>(slot) * n();
+  a.modes = born_modes_.at({hosts_[slot].re, hosts_[slot].im}).ptr;
+  a.tw = tw_born_.ptr;
+  a.basis = born_basis_.ptr;
+  a.state = gst_.ptr;
+  a.status = status_.ptr;
+  a.n = static_cast<int>(n());
+  a.dir = dir;
+  a.basis_smem = born_k_.basis_smem;
+  a.tol = in_.gmres_tol;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(born_k_.ctas);
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(born_k_.ctas);
+  cfg.blockDim = dim3(born_k_.threads);
+  cfg.dynamicSmemBytes = born_k_.smem;
+  cfg.stream = stream_;
+  cfg.attrs = attr;
+  cfg.numAttrs = born_k_.ctas > 1 ? 1 : 0;
+  void* args[] = {&a, &born_plan_.plan};
+  check_cuda(cudaLaunchKernelExC(&cfg, born_k_.fn, args), "k_born2d");
+  ++launches_;
+  born_graph_used_ = true;  // its error flag and counts are read at the end of the run
+}
+
 // Ŝ_m = F{V·F⁻¹{e^{i k_z s_m}(Ê⊥, Ê_z)}} into sources_ (cpp/src/solver.cpp:215-260).
 template <typename T>
 void PlaneSolver<T>::born_sources(const C* spec, int slot, int dir) {
@@ -1297,6 +1377,23 @@ void PlaneSolver<T>::sweeps(int iterations, const std::vector<int>& keep_slot, D
       const bool reflect = iterations > 0 && st.niface > 0;
       const C* add = (it > 0 && st.niface > 0) ? src_fwd_.ptr + 2 * st.iface_off : nullptr;
       const bool host = born && st.host_slot >= 0;
+      if (host && born_k_.fn) {
+        // the slab's step in the same launch where it is one transmission over all pixels
+        const bool one = st.pairs.size() == 1 && st.niface == 0;
+        const C* tab = nullptr;
+        if (one) {
+          const cd nr = index_of(st.pairs[0].first), ns = index_of(st.pairs[0].second);
+          tab = table(kFwdT, nr, ns);
+        } else {
+          step(p, false, reflect, e, next, reflect ? src_bwd_.ptr + 2 * st.iface_off : nullptr, add, true);
+        }
+        C* radiated = iterations > 0 ? born_bwd_.ptr + st.host_slot * n2 : nullptr;  // born_bwd[p + 1]
+        born_slab(st.host_slot, +1, one ? e : nullptr, tab, next,
+                  it > 0 ? born_fwd_.ptr + st.host_slot * n2 : nullptr, radiated, mask_.ptr);
+        std::swap(e, next);
+        if (last && keep_slot[p + 1] >= 0) copy(kept_f.ptr + keep_slot[p + 1] * n2, e);
+        continue;
+      }
       // 3D without Born slabs: each step leaves the next one's x transform (nothing else
       // touches the plane between two steps of a sweep)
       const bool fuse = !is2d() && !born;
@@ -1324,7 +1421,19 @@ void PlaneSolver<T>::sweeps(int iterations, const std::vector<int>& keep_slot, D
     if (last && keep_slot[nz] >= 0) copy(kept_b.ptr + keep_slot[nz] * n2, e);
     for (int p = nz; p > 0; --p) {
       const StepInfo& st = steps_[p - 1];
-      if (born && st.host_slot >= 0) {
+      if (born && st.host_slot >= 0 && born_k_.fn) {
+        C* radiated = born_fwd_.ptr + st.host_slot * n2;  // born_fwd[p]
+        const int before = p >= 2 ? steps_[p - 2].host_slot : -1;
+        const C* incoming = before >= 0 ? born_bwd_.ptr + before * n2 : nullptr;  // born_bwd[p − 1]
+        if (st.pairs.size() == 1 && st.niface == 0) {
+          const cd nr = index_of(st.pairs[0].second), ns = index_of(st.pairs[0].first);
+          born_slab(st.host_slot, -1, e, table(kBwdT, nr, ns), next, incoming, radiated, mask_.ptr);
+          std::swap(e, next);
+          if (last && keep_slot[p - 1] >= 0) copy(kept_b.ptr + keep_slot[p - 1] * n2, e);
+          continue;
+        }
+        born_slab(st.host_slot, -1, e, nullptr, e, nullptr, radiated, nullptr);  // R2 at plane p
+      } else if (born && st.host_slot >= 0) {
         fft_plane(e, spec_.ptr, 2, -1);
         born_sources(spec_.ptr, st.host_slot, -1);
         born_emission(st.host_slot, +1, born_fwd_.ptr + st.host_slot * n2);  // born_fwd[p]
@@ -1454,7 +1563,8 @@ void PlaneSolver<T>::run(const cd* field, int iterations, const std::int64_t* ke
     check_cuda(cudaMemcpy(&st, status_.ptr, sizeof(int), cudaMemcpyDeviceToHost), "status");
     if (st) {
       check_cuda(cudaMemsetAsync(status_.ptr, 0, sizeof(int), stream_), "status");
-      throw std::runtime_error("a bulk copy of the 3D slab step did not complete in time");
+      throw std::runtime_error(is2d() ? "an exchange of the Born slab did not complete in time"
+                                      : "a bulk copy of the 3D slab step did not complete in time");
     }
   }
 }

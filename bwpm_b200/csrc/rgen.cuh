@@ -131,12 +131,13 @@ __device__ __forceinline__ int mod_magic(int i, int L, unsigned magic) {
   return i - static_cast<int>(__umulhi(static_cast<unsigned>(i), magic)) * L;
 }
 
-// An inner stage of radix R over all threads of the block.
+// An inner stage of radix R over the gn threads of the line (gt: this thread's number).
 template <int DIR, int R, typename T>
 __device__ __forceinline__ void gmid(const cx<T>* in_buf, cx<T>* out_buf,
-                                     const Tw<T>* __restrict__ tw, int n, int L, unsigned magic) {
+                                     const Tw<T>* __restrict__ tw, int n, int L, unsigned magic, int gt,
+                                     int gn) {
   const int nb = n / R;
-  for (int i = threadIdx.x; i < nb; i += static_cast<int>(blockDim.x)) {
+  for (int i = gt; i < nb; i += gn) {
     const int k = mod_magic(i, L, magic);
     cx<T> u[R];
 #pragma unroll
@@ -151,11 +152,12 @@ __device__ __forceinline__ void gmid(const cx<T>* in_buf, cx<T>* out_buf,
 }
 
 // In-register transform of a line of n = E·nt points, plan radices (E, inner …, E); `phase` as
-// in rf::fft. Every thread of the block must call it; magic[s] belongs to plan.len[s].
+// in rf::fft. Every thread of the block must call it (t of the line's gn threads, nt of which own
+// values); magic[s] belongs to plan.len[s].
 template <int DIR, int E, typename T>
 __device__ __forceinline__ void gfft(cx<T> (&v)[E], cx<T>* b0, cx<T>* b1, int& phase, const FftPlan& plan,
                                      const unsigned* magic, const Tw<T>* __restrict__ tw, int t,
-                                     int nt) {
+                                     int nt, int gn) {
   const bool own = t < nt;
   {  // first stage: butterfly t of radix E, sub-length 1
     if (own) {
@@ -173,15 +175,15 @@ __device__ __forceinline__ void gfft(cx<T> (&v)[E], cx<T>* b0, cx<T>* b1, int& p
     const int L = plan.len[s];
     const Tw<T>* w = tw + plan.twoff[s];
     switch (plan.radix[s]) {
-      case 2: gmid<DIR, 2>(in, out, w, plan.n, L, magic[s]); break;
-      case 3: gmid<DIR, 3>(in, out, w, plan.n, L, magic[s]); break;
-      case 4: gmid<DIR, 4>(in, out, w, plan.n, L, magic[s]); break;
-      case 5: gmid<DIR, 5>(in, out, w, plan.n, L, magic[s]); break;
-      case 6: gmid<DIR, 6>(in, out, w, plan.n, L, magic[s]); break;
-      case 7: gmid<DIR, 7>(in, out, w, plan.n, L, magic[s]); break;
-      case 8: gmid<DIR, 8>(in, out, w, plan.n, L, magic[s]); break;
-      case 9: gmid<DIR, 9>(in, out, w, plan.n, L, magic[s]); break;
-      case 10: gmid<DIR, 10>(in, out, w, plan.n, L, magic[s]); break;
+      case 2: gmid<DIR, 2>(in, out, w, plan.n, L, magic[s], t, gn); break;
+      case 3: gmid<DIR, 3>(in, out, w, plan.n, L, magic[s], t, gn); break;
+      case 4: gmid<DIR, 4>(in, out, w, plan.n, L, magic[s], t, gn); break;
+      case 5: gmid<DIR, 5>(in, out, w, plan.n, L, magic[s], t, gn); break;
+      case 6: gmid<DIR, 6>(in, out, w, plan.n, L, magic[s], t, gn); break;
+      case 7: gmid<DIR, 7>(in, out, w, plan.n, L, magic[s], t, gn); break;
+      case 8: gmid<DIR, 8>(in, out, w, plan.n, L, magic[s], t, gn); break;
+      case 9: gmid<DIR, 9>(in, out, w, plan.n, L, magic[s], t, gn); break;
+      case 10: gmid<DIR, 10>(in, out, w, plan.n, L, magic[s], t, gn); break;
       default: break;  // the host plans inner radices 2 to 10 only
     }
     __syncthreads();
