@@ -33,7 +33,7 @@ namespace {
 constexpr int kClassThreads[] = {64, 128, 256, 512};
 constexpr int kGenericClasses = 4;
 constexpr int kMaxFixedLengths = 28;
-constexpr int kMaxRt = 12;
+constexpr int kMaxRt = 20;
 constexpr int kRtBase = kGenericClasses + kMaxFixedLengths;  // classes of the run-time-length kernels
 constexpr int kNumClasses = kRtBase + kMaxRt;  // [4, kRtBase): fixed lengths, then E values
 constexpr int kTuneScale = 4;     // autotuning runs keep 1/kTuneScale of every chain
@@ -60,8 +60,20 @@ int fixed_length_index(int n) {
 // Radices of a length n for a run-time-length kernel with E values per thread: the powers of two
 // as 8s (4s, 2s) when E allows, then 3s and 5s; empty if n has another prime factor. Stages
 // whose radix does not divide E run as gather stages (rgen.cuh).
-std::vector<int> rt_radices(int n, int e) {
+std::vector<int> rt_radices(int n, const RtVariant& rv) {
+  const int e = rv.e;
   std::vector<int> r;
+  if (rv.equal_outer) {  // (E, inner radices, E)
+    if (n % (e * e)) return {};
+    for (int p : {7, 11, 13})  // 2, 3 and 5 only, as the other run-time kernels
+      if (n % p == 0) return {};
+    std::vector<int> inner;
+    if (chain_inner(n / (e * e), n, (n / e + 31) / 32 * 32, 10, inner) >= 1e29) return {};
+    r.push_back(e);
+    r.insert(r.end(), inner.begin(), inner.end());
+    r.push_back(e);
+    return r;
+  }
   int m = n, twos = 0;
   while (m % 2 == 0) {
     m /= 2;
@@ -99,15 +111,22 @@ int rt_choice(int n) {
   const int forced_e = force ? std::atoi(force) : 0;
   for (std::size_t i = 0; i < rv.size(); ++i) {
     const int e = rv[i].e;
-    const bool wide = rv[i].max_threads > rg::rt_max_threads(e);
+    const bool outer = rv[i].equal_outer;
+    const bool wide = !outer && rv[i].max_threads > rg::rt_max_threads(e);
     if (n % e || n / e > rv[i].max_threads || (wide && n / e <= rg::rt_max_threads(e))) continue;
-    const std::vector<int> r = rt_radices(n, e);
+    if (!outer && best >= 0 && rv[best].equal_outer) break;  // listed first, and always the faster
+    const std::vector<int> r = rt_radices(n, rv[i]);
     if (r.empty()) continue;
     if (e == forced_e) return static_cast<int>(i);
     // a stage costs about (8 + E) value-times per thread (E values plus fixed overhead), twice
-    // for a gather stage
+    // for a gather stage; with equal outer radices the inner stages as chain_inner counts them
     double score = 0;
-    for (int x : r) score += (e % x == 0 ? 1.0 : 2.0) * (8.0 + e);
+    if (outer) {
+      std::vector<int> inner;
+      score = 2 * (14.0 + e) + chain_inner(n / (e * e), n, (n / e + 31) / 32 * 32, 10, inner);
+    } else {
+      for (int x : r) score += (e % x == 0 ? 1.0 : 2.0) * (8.0 + e);
+    }
     if (wide) score *= 1.2;
     if (score < best_score - 1e-9) {
       best_score = score;
@@ -582,7 +601,7 @@ void Batch2DImpl::prepare() {
       continue;
     }
     const int rt = rt_choice(n);
-    HostPlan hp = rt >= 0 ? make_plan_radices(n, rt_radices(n, rt_variants()[rt].e)) : make_plan(n);
+    HostPlan hp = rt >= 0 ? make_plan_radices(n, rt_radices(n, rt_variants()[rt])) : make_plan(n);
     const int base = static_cast<int>(tw.size());
     for (auto& t : twiddles_for<float>(hp)) tw.push_back(t);
     for (int st = 0; st < hp.plan.nstages; ++st) hp.plan.twoff[st] += base;

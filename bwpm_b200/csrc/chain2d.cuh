@@ -22,6 +22,7 @@
 #include <cstdlib>
 
 #include "chain2d.hpp"
+#include "plan.hpp"
 #include "plane_kernels.cuh"
 #include "resident2d.cuh"
 #include "rgen.cuh"
@@ -376,29 +377,6 @@ inline void chain_runtime(std::vector<ChainRuntime>& v) {
   v.push_back({E, 256, (const void*)k_chain2d<ch::RuntimeLine<T, E, 256>>});
   v.push_back({E, 384, (const void*)k_chain2d<ch::RuntimeLine<T, E, 384>>});
   v.push_back({E, 512, (const void*)k_chain2d<ch::RuntimeLine<T, E, 512>>});
-}
-
-// Plan (E, inner radices, E) of length n: the inner radices (10 to 2) with the smallest estimate
-// over their stages for nt threads; empty when E² does not divide n or a prime above 7 is left.
-// A stage costs about 6 value-times of latency per round of butterflies beside its values.
-inline double chain_inner(int m, int n, int nthr, int max_radix, std::vector<int>& out) {
-  if (m == 1) return 0.0;
-  double best = 1e30;
-  std::vector<int> pick;
-  for (int r = std::min(max_radix, 10); r >= 2; --r) {
-    if (m % r) continue;
-    std::vector<int> rest;
-    const double tail = chain_inner(m / r, n, nthr, r, rest);
-    const double rounds = (n / r + nthr - 1) / nthr;
-    const double cost = tail + 8.0 + rounds * (6.0 + r);
-    if (cost < best - 1e-9) {
-      best = cost;
-      pick = {r};
-      pick.insert(pick.end(), rest.begin(), rest.end());
-    }
-  }
-  out = pick;
-  return best;
 }
 
 // The run-time kernel of length n: the E (E² divides n, n/E within the thread limit) with the

@@ -1,6 +1,7 @@
 // Host-side FFT planning: factorisation into radices, thread requirement and FP64 twiddles.
 #pragma once
 
+#include <algorithm>
 #include <cmath>
 #include <string>
 #include <vector>
@@ -94,6 +95,29 @@ inline HostPlan make_plan_radices(int n, const std::vector<int>& radices) {
   if (hp.twiddles.empty()) hp.twiddles.push_back(cd{1.0, 0.0});
   p.ntw = static_cast<int>(hp.twiddles.size());
   return hp;
+}
+
+// Plan (E, inner radices, E) of length n: the inner radices (10 to 2) with the smallest estimate
+// over their stages for nt threads; empty when E² does not divide n or a prime above 7 is left.
+// A stage costs about 6 value-times of latency per round of butterflies beside its values.
+inline double chain_inner(int m, int n, int nthr, int max_radix, std::vector<int>& out) {
+  if (m == 1) return 0.0;
+  double best = 1e30;
+  std::vector<int> pick;
+  for (int r = std::min(max_radix, 10); r >= 2; --r) {
+    if (m % r) continue;
+    std::vector<int> rest;
+    const double tail = chain_inner(m / r, n, nthr, r, rest);
+    const double rounds = (n / r + nthr - 1) / nthr;
+    const double cost = tail + 8.0 + rounds * (6.0 + r);
+    if (cost < best - 1e-9) {
+      best = cost;
+      pick = {r};
+      pick.insert(pick.end(), rest.begin(), rest.end());
+    }
+  }
+  out = pick;
+  return best;
 }
 
 // Threads needed so that every stage fits its register staging of EPT values per thread

@@ -31,6 +31,16 @@ __device__ __forceinline__ int pad(int a) { return a + (a >> (sizeof(T) == sizeo
 template <typename T = float>
 __host__ __device__ constexpr int padded(int n) { return n + n / (sizeof(T) == sizeof(double) ? 8 : 16) + 1; }
 
+// pad(pos + r·STRIDE) given b = pad(pos): a constant step where STRIDE is whole padding blocks.
+template <int STRIDE, typename T>
+__device__ __forceinline__ int pad_step(int b, int pos, int r) {
+  constexpr int blk = sizeof(T) == sizeof(double) ? 8 : 16;
+  if constexpr (STRIDE % blk == 0)
+    return b + r * (STRIDE + STRIDE / blk);
+  else
+    return pad<T>(pos + r * STRIDE);
+}
+
 // x·exp(DIR·2πi·e/16) with exact (±1, ±i) cases and split constants otherwise.
 template <int DIR, int EXP>
 __device__ __forceinline__ cf w16mul(cf x) {
@@ -205,8 +215,9 @@ __device__ __forceinline__ void stage(cx<T> (&v)[N / NT], cx<T>* buf, const Tw<T
       for (int r = 0; r < R; ++r) v[j + r * K] = u[r];
     } else {
       const int base = (i - k) * R + k;
+      const int pb = pad<T>(base);
 #pragma unroll
-      for (int r = 0; r < R; ++r) buf[pad<T>(base + r * L)] = u[r];
+      for (int r = 0; r < R; ++r) buf[pad_step<L, T>(pb, base, r)] = u[r];
     }
     // compiler-only fence: one butterfly's twiddles and temporaries are dead before the next
     // butterfly's loads are issued (keeps the live registers of a stage at one butterfly)
@@ -214,8 +225,9 @@ __device__ __forceinline__ void stage(cx<T> (&v)[N / NT], cx<T>* buf, const Tw<T
   }
   if constexpr (!LAST) {
     __syncthreads();
+    const int pt = pad<T>(t);
 #pragma unroll
-    for (int m = 0; m < E; ++m) v[m] = buf[pad<T>(t + m * NT)];
+    for (int m = 0; m < E; ++m) v[m] = buf[pad_step<NT, T>(pt, t, m)];
   }
 }
 
@@ -267,16 +279,6 @@ __device__ __forceinline__ void stages(cx<T> (&v)[N / NT], cx<T>* b0, cx<T>* b1,
   if constexpr (!last) stages<DIR, N, NT, L * R, OFF + L * (R - 1), Rest...>(v, b0, b1, phase, tw, t);
 }
 
-// In-register transform of the owned values (DIR −1 forward, +1 inverse unnormalised).
-// `phase` selects the exchange buffer and must be uniform across the block; the buffer it
-// points to after the transform is free for the caller (no thread still reads it).
-template <int DIR, int N, int NT, int... Rs, typename T>
-__device__ __forceinline__ void fft(cx<T> (&v)[N / NT], cx<T>* b0, cx<T>* b1, int& phase,
-                                   const Tw<T>* __restrict__ tw, int t, Radices<Rs...>) {
-  static_assert((1 * ... * Rs) == N, "radices must multiply to N");
-  stages<DIR, N, NT, 1, 0, Rs...>(v, b0, b1, phase, tw, t);
-}
-
 // ---- transforms whose inner stages take any radix -----------------------------------------------
 //
 // The first and the last stage's radix divides E, so the transform still goes registers to
@@ -297,12 +299,13 @@ __device__ __forceinline__ void gstage(cx<T> (&v)[N / NT], const cx<T>* in_buf, 
     if (NB % NT == 0 || i < NB) {
       const int k = i % L;
       cx<T> u[R];
+      const int pi = pad<T>(i);
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         if constexpr (FIRST)
           u[r] = v[j + r * K];
         else
-          u[r] = in_buf[pad<T>(i + r * NB)];
+          u[r] = in_buf[pad_step<NB, T>(pi, i, r)];
       }
       if constexpr (L > 1) {
 #pragma unroll
@@ -314,8 +317,9 @@ __device__ __forceinline__ void gstage(cx<T> (&v)[N / NT], const cx<T>* in_buf, 
         for (int r = 0; r < R; ++r) v[j + r * K] = u[r];
       } else {
         const int base = (i - k) * R + k;
+        const int pb = pad<T>(base);
 #pragma unroll
-        for (int r = 0; r < R; ++r) out_buf[pad<T>(base + r * L)] = u[r];
+        for (int r = 0; r < R; ++r) out_buf[pad_step<L, T>(pb, base, r)] = u[r];
       }
     }
     asm volatile("" ::: "memory");
@@ -341,6 +345,22 @@ __device__ __forceinline__ void gfft(cx<T> (&v)[N / NT], cx<T>* b0, cx<T>* b1, i
                                      const Tw<T>* __restrict__ tw, int t, Radices<Rs...>) {
   static_assert((1 * ... * Rs) == N, "radices must multiply to N");
   gstages<DIR, N, NT, 1, 0, true, Rs...>(v, b0, b1, phase, tw, t);
+}
+
+// In-register transform of the owned values (DIR −1 forward, +1 inverse unnormalised).
+// `phase` selects the exchange buffer and must be uniform across the block; the buffer it
+// points to after the transform is free for the caller (no thread still reads it).
+template <int DIR, int N, int NT, int... Rs, typename T>
+__device__ __forceinline__ void fft(cx<T> (&v)[N / NT], cx<T>* b0, cx<T>* b1, int& phase,
+                                   const Tw<T>* __restrict__ tw, int t, Radices<Rs...>) {
+  static_assert((1 * ... * Rs) == N, "radices must multiply to N");
+  constexpr int E = N / NT;
+  constexpr int r[] = {Rs...};
+  constexpr bool all = ((E % Rs == 0) && ...);
+  if constexpr (!all && E % r[0] == 0 && E % r[sizeof...(Rs) - 1] == 0)
+    gfft<DIR, N, NT>(v, b0, b1, phase, tw, t, Radices<Rs...>{});  // inner radices that E does not hold
+  else
+    stages<DIR, N, NT, 1, 0, Rs...>(v, b0, b1, phase, tw, t);
 }
 
 }  // namespace rf

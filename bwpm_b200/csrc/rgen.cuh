@@ -227,16 +227,27 @@ __device__ __forceinline__ double flux(const cf (&v)[E], const double* w, double
   return total;
 }
 
+// The line's transform: rg::gfft (G) or rg::fft.
+template <int DIR, int E, bool G>
+__device__ __forceinline__ void line_fft(cf (&v)[E], cf* b0, cf* b1, int& phase, const FftPlan& plan,
+                                         const unsigned* magic, const Tw<float>* __restrict__ tw, int t,
+                                         int nt) {
+  if constexpr (G)
+    gfft<DIR, E>(v, b0, b1, phase, plan, magic, tw, t, nt, static_cast<int>(blockDim.x));
+  else
+    fft<DIR, E>(v, b0, b1, phase, plan, tw, t, nt);
+}
+
 // One slab step (cf. r2f_step: prefetched records and operator values, pair ids of the owned
 // pixels once per step, the next pass's operator values prefetched into L1, the first interface
 // round loaded before the forward transform; mk: the item's mask in shared memory, n hi then n lo
 // values, or null); every thread of the block calls it.
-template <int E>
+template <int E, bool G>
 __device__ __forceinline__ void step(cf (&v)[E], cf* S, cf (&out)[E], cf* b0, cf* b1, int& phase,
                                      const R2Item& it, const R2Step& st, const R2Pass& p0,
                                      const R2Pass& p1, R2Next& nx, int next_p, bool next_backward,
                                      bool backward, bool reflect, cf* store, const cf* add,
-                                     const float* mk, const FftPlan& plan,
+                                     const float* mk, const FftPlan& plan, const unsigned* magic,
                                      const Tw<float>* __restrict__ tw, int t, int nt) {
   constexpr int EW = (E + 3) / 4;
   const int n = it.n, nthr = static_cast<int>(blockDim.x);
@@ -260,13 +271,13 @@ __device__ __forceinline__ void step(cf (&v)[E], cf* S, cf (&out)[E], cf* b0, cf
         tl[k] = m[n + t + k * nt];
       }
     }
-    fft<-1, E>(v, b0, b1, phase, plan, tw, t, nt);
+    line_fft<-1, E, G>(v, b0, b1, phase, plan, magic, tw, t, nt);
     if (next_p >= 0) r2_next_passes(nx, it, next_backward);
     if (own) {
 #pragma unroll
       for (int k = 0; k < E; ++k) v[k] = pmul(v[k], th[k], tl[k]);
     }
-    fft<+1, E>(v, b0, b1, phase, plan, tw, t, nt);
+    line_fft<+1, E, G>(v, b0, b1, phase, plan, magic, tw, t, nt);
     if (own && mk) {
 #pragma unroll
       for (int k = 0; k < E; ++k) {
@@ -290,7 +301,7 @@ __device__ __forceinline__ void step(cf (&v)[E], cf* S, cf (&out)[E], cf* b0, cf
         prefetch_l1(m + n + t + k * nt);
       }
     }
-    fft<-1, E>(v, b0, b1, phase, plan, tw, t, nt);
+    line_fft<-1, E, G>(v, b0, b1, phase, plan, magic, tw, t, nt);
     if (next_p >= 0) r2_next_passes(nx, it, next_backward);
     const int pid0 = (pid && own_if) ? pid[q0] : 0;
     if (own) {
@@ -318,7 +329,7 @@ __device__ __forceinline__ void step(cf (&v)[E], cf* S, cf (&out)[E], cf* b0, cf
           if ((k & 3) == 3) asm volatile("" ::: "memory");
         }
       }
-      fft<+1, E>(v, b0, b1, phase, plan, tw, t, nt);
+      line_fft<+1, E, G>(v, b0, b1, phase, plan, magic, tw, t, nt);
       if (!cur.refl) {
         if (own) {
 #pragma unroll
@@ -390,13 +401,15 @@ __host__ __device__ constexpr std::size_t rt_smem_bytes(int n) {
 // the thread limit (and so the register budget) of the instance; 512 for a small E is the wide
 // form for lines whose n/E exceeds the default limit (128 registers: it spills, but a line of
 // 4050 points then runs on 450 threads with E = 9 instead of 135 with E = 30: 57 → 36 µs a step).
-template <int E, int NTMAX = rg::rt_max_threads(E)>
+// G: plans with equal outer radices (rg::gfft).
+template <int E, int NTMAX = rg::rt_max_threads(E), bool G = false>
 __global__ void __launch_bounds__(NTMAX, 1)
     k_resident2d_rt(const R2Item* __restrict__ items, int nitems, int* queue, R2Shared sh) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_item;
   __shared__ double s_red[512];
   __shared__ FftPlan s_plan;
+  __shared__ unsigned s_magic[kMaxStages];
   const int t = threadIdx.x;
   int phase = 0;
   for (;;) {
@@ -411,7 +424,10 @@ __global__ void __launch_bounds__(NTMAX, 1)
     const int base = sh.plans[it.plan].twoff[0];
     if (t == 0) {
       s_plan = sh.plans[it.plan];
-      for (int st = 0; st < s_plan.nstages; ++st) s_plan.twoff[st] -= base;
+      for (int st = 0; st < s_plan.nstages; ++st) {
+        s_plan.twoff[st] -= base;
+        s_magic[st] = 0xffffffffu / static_cast<unsigned>(s_plan.len[st]) + 1u;
+      }
       it.clock[0] = global_ns();
     }
     for (int i = t; i < n - 1; i += static_cast<int>(blockDim.x)) tws[i] = sh.twiddles[base + i];
@@ -433,7 +449,7 @@ __global__ void __launch_bounds__(NTMAX, 1)
 #pragma unroll
       for (int m = 0; m < E; ++m) v[m] = it.input[t + m * nt];
     }
-    rg::fft<-1, E>(v, b0, b1, phase, plan, tws, t, nt);
+    rg::line_fft<-1, E, G>(v, b0, b1, phase, plan, s_magic, tws, t, nt);
     {
       const double pin = rg::flux<E>(v, it.w_in, s_red, t, nt);
       if (t == 0) it.energy[2 * iters] = pin;
@@ -459,8 +475,8 @@ __global__ void __launch_bounds__(NTMAX, 1)
         const bool has_add = st.niface > 0 && (backward || iter > 0);
         cf* store = (backward ? it.src_fwd : it.src_bwd) + st.iface;
         const cf* add = has_add ? (backward ? it.src_bwd : it.src_fwd) + st.iface : nullptr;
-        rg::step<E>(v, S, out, b0, b1, phase, it, st, p0, p1, nx, next_p, next_backward,
-                    backward, reflect, store, add, mk, plan, tws, t, nt);
+        rg::step<E, G>(v, S, out, b0, b1, phase, it, st, p0, p1, nx, next_p, next_backward,
+                    backward, reflect, store, add, mk, plan, s_magic, tws, t, nt);
       }
       cf* dst = backward ? it.reflected : it.transmitted;
       if (own) {
@@ -472,7 +488,7 @@ __global__ void __launch_bounds__(NTMAX, 1)
 #pragma unroll
         for (int m = 0; m < E; ++m) out[m] = v[m];
       }
-      rg::fft<-1, E>(out, b0, b1, phase, plan, tws, t, nt);
+      rg::line_fft<-1, E, G>(out, b0, b1, phase, plan, s_magic, tws, t, nt);
       const double fl = rg::flux<E>(out, backward ? it.w_in : it.w_out, s_red, t, nt);
       if (t == 0) it.energy[2 * iter + (backward ? 1 : 0)] = fl;
     }

@@ -28,6 +28,7 @@ struct RtVariant {
   int e;
   const void* fn;
   int max_threads;  // the instance's thread limit (rg::rt_max_threads(e), or 512: wide form)
+  bool equal_outer; // plans (E, inner radices, E) for lengths that E² divides (rg::gfft)
 };
 const std::vector<RtVariant>& rt_variants();
 

@@ -16,14 +16,15 @@ FixedVariant fixed() {
 
 void add_variants_small(std::vector<FixedVariant>& v) {
   // per length, only variants that no other variant beats in both per-step latency and SM time
-  // (measured on a B200: 1 item, tilted slab, 400 slabs)
-  v.push_back(fixed<256, 32, 8, 8, 4>());
-  v.push_back(fixed<384, 32, 4, 4, 4, 3, 2>());
-  v.push_back(fixed<512, 64, 8, 8, 8>());
-  v.push_back(fixed<768, 64, 4, 4, 4, 4, 3>());
-  v.push_back(fixed<1024, 128, 8, 8, 8, 2>());
-  v.push_back(fixed<1536, 192, 8, 8, 8, 3>());  // radix 3 as a gather stage
-  v.push_back(fixed<1536, 128, 4, 4, 4, 4, 2, 3>());
+  // (measured on a B200: 1 item, tilted slab, 400 slabs; µs per step, the variant replaced in
+  // brackets). Four values a thread on twice the warps win up to 512 points, inner stages of any
+  // radix (rf::gfft) at the lengths with a factor 3.
+  v.push_back(fixed<256, 64, 4, 4, 4, 4>());    // 0.74 (8·8·4 on 32 threads: 0.92)
+  v.push_back(fixed<384, 96, 4, 6, 4, 4>());    // 0.89 (4·4·4·3·2 on 32 threads: 2.0)
+  v.push_back(fixed<512, 128, 4, 8, 4, 4>());   // 1.02 (8·8·8 on 64 threads: 1.11)
+  v.push_back(fixed<768, 96, 8, 12, 8>());      // 1.47 (4·4·4·4·3 on 64 threads: 2.4)
+  v.push_back(fixed<1024, 128, 8, 8, 8, 2>());  // 1.74 (4·8·8·4 on 256 threads: 2.1)
+  v.push_back(fixed<1536, 192, 8, 4, 6, 8>());  // 3.0 (8·8·8·3 on 192 threads: 3.6)
 }
 
 const std::vector<FixedVariant>& fixed_variants() {
