@@ -64,14 +64,9 @@ std::vector<int> rt_radices(int n, const RtVariant& rv) {
   const int e = rv.e;
   std::vector<int> r;
   if (rv.equal_outer) {  // (E, inner radices, E)
-    if (n % (e * e)) return {};
     for (int p : {7, 11, 13})  // 2, 3 and 5 only, as the other run-time kernels
       if (n % p == 0) return {};
-    std::vector<int> inner;
-    if (chain_inner(n / (e * e), n, (n / e + 31) / 32 * 32, 10, inner) >= 1e29) return {};
-    r.push_back(e);
-    r.insert(r.end(), inner.begin(), inner.end());
-    r.push_back(e);
+    equal_outer_plan(n, e, (n / e + 31) / 32 * 32, r);
     return r;
   }
   int m = n, twos = 0;
@@ -119,11 +114,11 @@ int rt_choice(int n) {
     if (r.empty()) continue;
     if (e == forced_e) return static_cast<int>(i);
     // a stage costs about (8 + E) value-times per thread (E values plus fixed overhead), twice
-    // for a gather stage; with equal outer radices the inner stages as chain_inner counts them
+    // for a gather stage; with equal outer radices equal_outer_plan's cost
     double score = 0;
     if (outer) {
-      std::vector<int> inner;
-      score = 2 * (14.0 + e) + chain_inner(n / (e * e), n, (n / e + 31) / 32 * 32, 10, inner);
+      std::vector<int> radices;
+      score = equal_outer_plan(n, e, (n / e + 31) / 32 * 32, radices);
     } else {
       for (int x : r) score += (e % x == 0 ? 1.0 : 2.0) * (8.0 + e);
     }

@@ -21,12 +21,10 @@
 
 #include <algorithm>
 
-#include <cooperative_groups.h>
-
 #include "born2d.hpp"
 #include "born_kernels.cuh"
 #include "chain2d.cuh"
-#include "cluster2d.cuh"
+#include "cline.cuh"
 #include "gmres_kernels.cuh"
 
 namespace bwpm {
@@ -96,134 +94,6 @@ constexpr int kBornVectors = kGmresRestart + 4;
 
 namespace born {
 
-namespace cg = cooperative_groups;
-
-__device__ __forceinline__ void st_async16(unsigned raddr, cd v, unsigned rmbar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];"
-               :: "r"(raddr), "l"(__double_as_longlong(v.re)), "l"(__double_as_longlong(v.im)), "r"(rmbar)
-               : "memory");
-}
-__device__ __forceinline__ void send(unsigned raddr, cd v, unsigned rmbar) { st_async16(raddr, v, rmbar); }
-__device__ __forceinline__ void send(unsigned raddr, cf v, unsigned rmbar) { r2c::st_async(raddr, v, rmbar); }
-
-// The CTA's exchange state: two receive buffers used in turn, one mbarrier each (see "exchanges
-// through distributed shared memory" in cluster2d.cuh: a buffer is written again only after every
-// peer has received the exchange between). Fields and inner products take turns on it alike.
-struct Xch {
-  unsigned char* base;   // the buffers, `len` bytes each
-  unsigned len, mbar0;   // and their mbarriers, 8 bytes apart (shared-window address)
-  unsigned parity;
-  int cur;
-  int* status;
-  __device__ __forceinline__ unsigned char* buf() const { return base + cur * len; }
-  __device__ __forceinline__ unsigned mbar() const { return mbar0 + 8 * cur; }
-  __device__ __forceinline__ void open(unsigned bytes) {
-    if (threadIdx.x == 0) r2c::mbar_expect(mbar(), bytes);
-  }
-  __device__ __forceinline__ void wait() {
-    r2c::Exchange e;  // one exchange on the current buffer (r2c::xwait: bounded)
-    e.mbar[0] = mbar();
-    e.parity = (parity >> cur) & 1u;
-    e.cur = 0;
-    e.status = status;
-    r2c::xwait(e);
-    parity ^= 1u << cur;
-    cur ^= 1;
-  }
-};
-
-// A component's line over the cluster. Thread t of the group owns the real-space points
-// C·(t + m·nt) + c (m < E) and the spectral points c·MB + t + b·nt + M·k2 (b < SB, k2 < C).
-template <class Inner, int C>
-struct Line {
-  using T = typename Inner::T;
-  static constexpr int E = Inner::E, SB = (E + C - 1) / C, S = SB * C, ES = S > E ? S : E;
-  Inner in;
-  int rank, group, M, MB, mb;  // mb: spectral block of this CTA
-  const Tw<T>*xf, *xi;         // cross twiddles: w_N^{rank·k1}; block entries [d·MB + k1l] of w_N^{d·k1}
-  __device__ __forceinline__ int pos(int m) const { return C * in.pos(m) + rank; }
-  __device__ __forceinline__ bool own() const { return in.own(); }
-  __device__ __forceinline__ int k1l(int b) const { return in.t + b * in.threads(); }
-  __device__ __forceinline__ bool sown(int s) const { return in.own() && k1l(s % SB) < mb; }
-  __device__ __forceinline__ int spos(int s) const { return rank * MB + k1l(s % SB) + M * (s / SB); }
-  // own slot in a CTA-local array of M spectral values
-  __device__ __forceinline__ int slot(int s) const { return k1l(s % SB) + MB * (s / SB); }
-  __device__ __forceinline__ cx<T>* recv(const Xch& x) const {
-    return reinterpret_cast<cx<T>*>(x.buf()) + group * C * MB;
-  }
-
-  // real → spectrum; bytes: what this CTA receives over all groups
-  __device__ __forceinline__ void forward(cx<T> (&v)[ES], Xch& x, unsigned bytes) {
-    cx<T> u[E];
-#pragma unroll
-    for (int m = 0; m < E; ++m) u[m] = v[m];
-    in.template fft<-1>(u);
-    if constexpr (C == 1) {
-#pragma unroll
-      for (int m = 0; m < E; ++m) v[m] = u[m];
-    } else {
-      cx<T>* buf = recv(x);
-      const unsigned base = r2c::smem_u32(buf), mb0 = x.mbar();
-      x.open(bytes);
-      if (own()) {
-#pragma unroll
-        for (int m = 0; m < E; ++m) {
-          const int k1 = in.pos(m), dst = k1 / MB;
-          const unsigned off = static_cast<unsigned>(rank * MB + k1 - dst * MB) * sizeof(cx<T>);
-          send(r2c::mapa(base, dst) + off, rank == 0 ? u[m] : twmul<-1>(u[m], xf[k1]), r2c::mapa(mb0, dst));
-        }
-      }
-      x.wait();
-#pragma unroll
-      for (int b = 0; b < SB; ++b) {
-        cx<T> d[C];
-        if (in.own() && k1l(b) < mb) {
-#pragma unroll
-          for (int r = 0; r < C; ++r) d[r] = buf[r * MB + k1l(b)];
-          rf::dft<-1, C>(d);
-#pragma unroll
-          for (int r = 0; r < C; ++r) v[r * SB + b] = d[r];
-        }
-      }
-    }
-  }
-
-  // spectrum → real (unnormalised)
-  __device__ __forceinline__ void inverse(cx<T> (&v)[ES], Xch& x, unsigned bytes) {
-    cx<T> u[E];
-    if constexpr (C == 1) {
-#pragma unroll
-      for (int m = 0; m < E; ++m) u[m] = v[m];
-    } else {
-      cx<T>* buf = recv(x);
-      const unsigned base = r2c::smem_u32(buf), mb0 = x.mbar();
-      x.open(bytes);
-#pragma unroll
-      for (int b = 0; b < SB; ++b) {
-        if (in.own() && k1l(b) < mb) {
-          cx<T> d[C];
-#pragma unroll
-          for (int r = 0; r < C; ++r) d[r] = v[r * SB + b];
-          rf::dft<+1, C>(d);
-          const unsigned off = static_cast<unsigned>(rank * MB + k1l(b)) * sizeof(cx<T>);
-#pragma unroll
-          for (int r = 0; r < C; ++r)
-            send(r2c::mapa(base, r) + off, r == 0 ? d[r] : twmul<+1>(d[r], xi[r * MB + k1l(b)]),
-                 r2c::mapa(mb0, r));
-        }
-      }
-      x.wait();
-      if (own()) {
-#pragma unroll
-        for (int m = 0; m < E; ++m) u[m] = buf[in.pos(m)];
-      }
-    }
-    in.template fft<+1>(u);
-#pragma unroll
-    for (int m = 0; m < E; ++m) v[m] = u[m];
-  }
-};
-
 // GMRES scalars of a CTA (each CTA computes the same values).
 struct Scalars {
   cd h[(kGmresRestart + 1) * kGmresRestart];
@@ -244,7 +114,7 @@ __global__ void __launch_bounds__(born_threads<Inner>(), 1)
     k_born2d(const __grid_constant__ BornSlab<typename Inner::T> a, const __grid_constant__ FftPlan plan) {
   using T = typename Inner::T;
   using V = cx<T>;
-  using L = born::Line<Inner, C>;
+  using L = cl::Line<Inner, C>;
   constexpr int E = L::E, S = L::S, ES = L::ES;
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ FftPlan s_plan;
@@ -255,7 +125,7 @@ __global__ void __launch_bounds__(born_threads<Inner>(), 1)
   const int tid = threadIdx.x, group_threads = blockDim.x / 3;
   const int comp = tid / group_threads, t = tid - comp * group_threads;
   int rank = 0;
-  if constexpr (C > 1) rank = static_cast<int>(born::cg::this_cluster().block_rank());
+  if constexpr (C > 1) rank = static_cast<int>(cl::cg::this_cluster().block_rank());
   const int n = a.n, M = n / C, MB = (M + C - 1) / C, pm = rf::padded<T>(M);
   const int mb = max(0, min(MB, M - rank * MB));
   if (tid == 0) {
@@ -278,7 +148,7 @@ __global__ void __launch_bounds__(born_threads<Inner>(), 1)
   };
   V* lines = reinterpret_cast<V*>(take(3 * 2 * pm * sizeof(V)));
   const std::size_t recv = C > 1 ? 3 * C * MB * sizeof(V) : 0;
-  born::Xch x;
+  cl::Xch x;
   x.len = static_cast<unsigned>((recv > 256 ? recv : 256) + 15) / 16 * 16;
   x.base = take(2 * x.len);
   x.mbar0 = r2c::smem_u32(&s_mbar[0]);
@@ -312,7 +182,7 @@ __global__ void __launch_bounds__(born_threads<Inner>(), 1)
   const unsigned field_bytes = static_cast<unsigned>(3 * C * mb * sizeof(V));      // forward
   const unsigned inv_bytes = static_cast<unsigned>(3 * M * sizeof(V));             // inverse
   if constexpr (C > 1)
-    born::cg::this_cluster().sync();
+    cl::cg::this_cluster().sync();
   else
     __syncthreads();
   const bool own = ln.own();
@@ -356,7 +226,7 @@ __global__ void __launch_bounds__(born_threads<Inner>(), 1)
       if (tid < C) {  // thread d sends this CTA's sum to CTA d
         cd p{0.0, 0.0};
         for (int w = 0; w < warps; ++w) p = p + s_red[w];
-        born::st_async16(r2c::mapa(r2c::smem_u32(part), tid) + rank * sizeof(cd), p,
+        cl::st_async16(r2c::mapa(r2c::smem_u32(part), tid) + rank * sizeof(cd), p,
                          r2c::mapa(x.mbar(), tid));
       }
       x.wait();
@@ -621,7 +491,7 @@ __global__ void __launch_bounds__(born_threads<Inner>(), 1)
     a.state->applies += applies;
     if (err) a.state->err = 1;
   }
-  if constexpr (C > 1) born::cg::this_cluster().sync();  // no CTA leaves while a peer may still send
+  if constexpr (C > 1) cl::cg::this_cluster().sync();  // no CTA leaves while a peer may still send
 }
 
 // ---- host side ---------------------------------------------------------------------------------
@@ -655,12 +525,8 @@ inline bool born_fill(BornKernel& k, int n, int nt, std::vector<int> radices) {
 template <typename T, int E, int C>
 inline bool born_runtime(BornKernel& k, int n) {
   const int m = n / C;
-  if (m % (E * E)) return false;
-  std::vector<int> radices{E};
-  std::vector<int> inner;
-  if (chain_inner(m / (E * E), m, std::max(1, m / E), 10, inner) >= 1e29) return false;
-  radices.insert(radices.end(), inner.begin(), inner.end());
-  radices.push_back(E);
+  std::vector<int> radices;
+  if (equal_outer_plan(m, E, std::max(1, m / E), radices) >= 1e29) return false;
   return born_fill<T, ch::RuntimeLine<T, E, 384>, C>(k, n, m / E, radices);
 }
 

@@ -1,16 +1,19 @@
 // 2D chain kernels of the plane engine: every sweep of a 2D solve (nx = 1) in one launch.
 //
-// In 2D E_x and E_y are independent (k_x = 0 exactly), so a launch has two CTAs, one per
-// component, each running the whole run (forward and backward sweeps, all iterations,
-// cpp/src/solver.cpp:444-528) with its line in registers. The launch-per-step form they replace
-// (k_step2d) is bound by latency: a launch gap, a global round trip of the line and a shared-memory
-// transform with two barriers per stage for every step, on two SMs. Here a step is a register-
-// resident forward transform (rfft.cuh, rgen.cuh: one exchange and one barrier per stage), per
-// pass the operator product, the inverse transform and the epilogue (selection by pair id, mask,
+// In 2D E_x and E_y are independent (k_x = 0 exactly), so a launch has one CTA, or for long lines
+// one cluster, per component, which runs the whole run (forward and backward sweeps, all
+// iterations, cpp/src/solver.cpp:444-528) with its line in registers. The launch-per-step form it
+// replaces (k_step2d) is bound by latency: a launch gap, a global round trip of the line and a
+// shared-memory transform with two barriers per stage for every step, on two SMs. Here a step is a
+// register-resident forward transform (rfft.cuh, rgen.cuh: one exchange and one barrier per stage),
+// per pass the operator product, the inverse transform and the epilogue (selection by pair id, mask,
 // reflection gather), then the sparse sources; records of the next step load while the current
-// one computes, operator values are brought into L1 during the forward transform. Per step (200
-// slabs, tilted facet and mask, launch per step → chain): FP64 256 points 10.5 → 1.8 µs, 1024
-// 17.3 → 3.1, 2430 44.4 → 13.7, 4096 41.1 → 15.9; complex64 1024 14.3 → 2.7, 4096 31.0 → 13.4.
+// one computes, operator values are brought into L1 during the forward transform. A line on one SM
+// is bound by that SM's FP64 rate and issue from ≈ 1000 points on, so longer lines are split over
+// up to eight CTAs (cline.cuh), at an exchange of ≈ 0.7 µs per transform. Per step (200 slabs,
+// tilted facet and mask; launch per step → one CTA → split): FP64 256 points 10.5 → 1.4 µs, 1024
+// 17.3 → 3.1 → 2.7, 2430 44.4 → 13.7 → 6.9, 4096 41.1 → 15.9 → 5.3, 8192 129 → 9.9 (split);
+// complex64 1024 14.3 → 2.7, 2430 26.0 → 11.9 → 7.3, 4096 31.0 → 13.4 → 5.9.
 //
 // A step that nothing acts on in real space (one pair, no mask, no sources to add, plane not
 // kept, not the last of its sweep) leaves its result in the spectrum: the inverse transform and
@@ -22,6 +25,7 @@
 #include <cstdlib>
 
 #include "chain2d.hpp"
+#include "cline.cuh"
 #include "plan.hpp"
 #include "plane_kernels.cuh"
 #include "resident2d.cuh"
@@ -45,10 +49,10 @@ struct ChainArgs {
   cx<T>* src_fwd;            // sources of the forward sweep (gathered by the backward one)
   cx<T>* src_bwd;
   const T* mask;             // (N) (FP32: N hi, then N lo values), or null
-  cx<T>* spec;               // (2, N) scratch for the spectrum where shared memory has no room
-  const Tw<T>* tw;
+  cx<T>* spec;               // scratch for the spectrum where shared memory has no room
+  const Tw<T>* tw;           // stage twiddles (of the part), split lines: then w_N^{c·k}
   int n, nz, iterations;
-  int ntw;                   // stage twiddles
+  int* status;               // set to 1 when an exchange of a split line gave up
   int tw_smem, mask_smem, spec_smem;
   T inv_n;                   // FP64: 1/N after an inverse transform (FP32 tables carry it)
 };
@@ -104,6 +108,54 @@ struct RuntimeLine {
   }
 };
 
+// A whole line on one CTA, or split over a cluster (cline.cuh): real-space values pos(m) (lpos: their
+// number within the CTA), spectral values spos(s) (sidx: their place in a CTA-local array).
+template <class Inner>
+struct Whole {
+  using T = typename Inner::T;
+  using In = Inner;
+  static constexpr int C = 1, E = Inner::E, S = E, ES = E;
+  Inner in;
+  __device__ __forceinline__ Whole(Inner i) : in(i) {}
+  __device__ __forceinline__ Inner& line() { return in; }
+  __device__ __forceinline__ bool own() const { return in.own(); }
+  __device__ __forceinline__ bool sown(int) const { return in.own(); }
+  __device__ __forceinline__ int pos(int m) const { return in.pos(m); }
+  __device__ __forceinline__ int lpos(int m) const { return in.pos(m); }
+  __device__ __forceinline__ int spos(int s) const { return in.pos(s); }
+  __device__ __forceinline__ int sidx(int s) const { return in.pos(s); }
+  __device__ __forceinline__ bool mine(int) const { return true; }
+  __device__ __forceinline__ int local(int q) const { return q; }
+  __device__ __forceinline__ void forward(cx<T> (&v)[ES]) { in.template fft<-1>(v); }
+  __device__ __forceinline__ void inverse(cx<T> (&v)[ES]) { in.template fft<+1>(v); }
+};
+
+template <class Inner, int C_>
+struct Split {
+  using T = typename Inner::T;
+  using In = Inner;
+  using L = cl::Line<Inner, C_>;
+  static constexpr int C = C_, E = L::E, S = L::S, ES = L::ES;
+  L ln;
+  cl::Xch x;
+  __device__ __forceinline__ Split(L l, cl::Xch xch) : ln(l), x(xch) {}
+  __device__ __forceinline__ Inner& line() { return ln.in; }
+  __device__ __forceinline__ bool own() const { return ln.own(); }
+  __device__ __forceinline__ bool sown(int s) const { return ln.sown(s); }
+  __device__ __forceinline__ int pos(int m) const { return ln.pos(m); }
+  __device__ __forceinline__ int lpos(int m) const { return ln.in.pos(m); }
+  __device__ __forceinline__ int spos(int s) const { return ln.spos(s); }
+  __device__ __forceinline__ int sidx(int s) const { return ln.slot(s); }
+  __device__ __forceinline__ bool mine(int q) const { return q % C == ln.rank; }
+  __device__ __forceinline__ int local(int q) const { return q / C; }
+  __device__ __forceinline__ void forward(cx<T> (&v)[ES]) {
+    ln.forward(v, x, static_cast<unsigned>(C * ln.mb * sizeof(cx<T>)));
+  }
+  __device__ __forceinline__ void inverse(cx<T> (&v)[ES]) {
+    ln.inverse(v, x, static_cast<unsigned>(ln.M * sizeof(cx<T>)));
+  }
+};
+
 // Operator value q of a pass: FP64 one value; FP32 hi, and lo three blocks of n further on.
 template <typename T>
 __device__ __forceinline__ cx<T> op(cx<T> u, const cx<T>* m, int q, int n) {
@@ -130,49 +182,91 @@ struct ChainNext {
   PassRec p0;
 };
 
-template <class Line>
-__global__ void __launch_bounds__(Line::kMaxThreads, 1)
-    k_chain2d(const __grid_constant__ ChainArgs<typename Line::T> a,
+template <class W>
+__global__ void __launch_bounds__(W::In::kMaxThreads, 1)
+    k_chain2d(const __grid_constant__ ChainArgs<typename W::T> a,
               const __grid_constant__ FftPlan plan) {
-  using T = typename Line::T;
+  using T = typename W::T;
   using C = cx<T>;
-  constexpr int E = Line::E, EW = (E + 3) / 4;
+  constexpr int E = W::E, S = W::S, ES = W::ES, EW = (E + 3) / 4, K = W::C;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ FftPlan s_plan;
   __shared__ unsigned s_magic[kMaxStages];
-  const int c = blockIdx.x, t = threadIdx.x, nthr = blockDim.x;
-  if constexpr (Line::kRuntime) {
-    if (t == 0) {
+  __shared__ alignas(8) unsigned long long s_mbar[2];
+  // K CTAs (a cluster) per component; M points per CTA, MB of them in its spectral block
+  const int c = blockIdx.x / K, rank = blockIdx.x - c * K, t = threadIdx.x, nthr = blockDim.x;
+  const int n = a.n, M = n / K, MB = (M + K - 1) / K, pn = rf::padded<T>(M);
+  if (t == 0) {
+    if constexpr (W::In::kRuntime) {
       s_plan = plan;
       for (int s = 0; s < plan.nstages; ++s)
         s_magic[s] = 0xffffffffu / static_cast<unsigned>(plan.len[s]) + 1u;
     }
-    __syncthreads();
+    if constexpr (K > 1) {
+      r2c::mbar_init(r2c::smem_u32(&s_mbar[0]), 1);
+      r2c::mbar_init(r2c::smem_u32(&s_mbar[1]), 1);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
   }
+  // two exchange lines; split lines: two receive buffers and the cross twiddles; then, where they
+  // fit, the stage twiddles, the mask (8 bytes a point in both types) and the spectrum of a
+  // multi-pass step
   C* lines = reinterpret_cast<C*>(smem_raw);
-  Line ln(s_plan, s_magic, a.n, a.tw, lines, t, nthr);
-  const int n = ln.n(), pn = rf::padded<T>(n);
-  const bool own = ln.own();
-  // beside the two exchange lines, where they fit: the stage twiddles, the mask (8 bytes a point
-  // in both types), the spectrum of a multi-pass step
   unsigned char* more = smem_raw + 2 * pn * sizeof(C);
-  if (a.tw_smem) {
-    Tw<T>* tws = reinterpret_cast<Tw<T>*>(more);
-    for (int i = t; i < a.ntw; i += nthr) tws[i] = a.tw[i];
-    ln.tw = tws;
-    more += a.ntw * sizeof(Tw<T>);
+  const Tw<T>* tws = a.tw;
+  Tw<T>*xfs = nullptr, *xis = nullptr;
+  cl::Xch x{};
+  if constexpr (K > 1) {
+    x.base = more;
+    x.len = static_cast<unsigned>(K * MB * sizeof(C));
+    x.mbar0 = r2c::smem_u32(&s_mbar[0]);
+    x.status = a.status;
+    more += 2 * x.len;
+    xfs = reinterpret_cast<Tw<T>*>(more);
+    xis = xfs + M;
+    more += (M + K * MB) * sizeof(Tw<T>);
+    const Tw<T>* xg = a.tw + (M - 1);
+    for (int i = t; i < M; i += nthr) xfs[i] = xg[static_cast<long long>(rank) * M + i];
+    for (int i = t; i < K * MB; i += nthr) {
+      const int d = i / MB, k1 = rank * MB + i - d * MB;
+      if (k1 < M) xis[i] = xg[static_cast<long long>(d) * M + k1];
+    }
   }
-  const T* mk = a.mask;
+  if (a.tw_smem) {
+    Tw<T>* s = reinterpret_cast<Tw<T>*>(more);
+    for (int i = t; i < M - 1; i += nthr) s[i] = a.tw[i];
+    tws = s;
+    more += (M - 1) * sizeof(Tw<T>);
+  }
+  const T* mk = a.mask;  // staged: indexed by the CTA's own numbering, lo parts M further on
   if (a.mask && a.mask_smem) {
     T* mask_s = reinterpret_cast<T*>(more);
-    constexpr int MV = sizeof(T) == sizeof(double) ? 1 : 2;  // mask values per point
-    for (int i = t; i < MV * n; i += nthr) mask_s[i] = a.mask[i];
+    for (int i = t; i < M; i += nthr) {
+      mask_s[i] = a.mask[K * i + rank];
+      if constexpr (sizeof(T) != sizeof(double)) mask_s[M + i] = a.mask[n + K * i + rank];
+    }
     mk = mask_s;
-    more += (8 * n + 15) / 16 * 16;
+    more += (8 * M + 15) / 16 * 16;
   }
-  C* S = a.spec_smem ? reinterpret_cast<C*>(more) : a.spec + static_cast<long long>(c) * n;
+  C* spec_line = a.spec_smem ? reinterpret_cast<C*>(more)
+                             : a.spec + static_cast<long long>(c * K + rank) * K * MB;
+  auto make = [&]() {
+    typename W::In in(s_plan, s_magic, M, tws, lines, t, nthr);
+    if constexpr (K > 1)
+      return W(typename W::L{in, rank, 0, M, MB, max(0, min(MB, M - rank * MB)), xfs, xis}, x);
+    else
+      return W(in);
+  };
   __syncthreads();
-  C v[E], out[E];
+  W ln = make();
+  auto& in = ln.line();
+  const bool own = ln.own();
+  const int mo = a.mask_smem ? M : n;  // distance of a mask's lo parts
+  if constexpr (K > 1)
+    cl::cg::this_cluster().sync();
+  else
+    __syncthreads();
+  C v[ES], out[E];
   const int sweeps = a.iterations > 0 ? 2 * a.iterations : 1;
   const int iters = a.iterations > 0 ? a.iterations : 1;
   const int eoff = c == 0 ? 0 : 2 * n;  // m00 for E_x, m11 for E_y
@@ -223,46 +317,44 @@ __global__ void __launch_bounds__(Line::kMaxThreads, 1)
         for (int m = 0; m < E; ++m)
           pw[m >> 2] |= static_cast<std::uint32_t>(pid[ln.pos(m)]) << (8 * (m & 3));
       }
-      if (own) {
+      {
         const C* m0 = static_cast<const C*>(cur.tab) + eoff;
 #pragma unroll
-        for (int m = 0; m < E; ++m) ch::op_prefetch(m0, ln.pos(m), n);
+        for (int s2 = 0; s2 < S; ++s2)
+          if (ln.sown(s2)) ch::op_prefetch(m0, ln.spos(s2), n);
       }
-      if (!spectral) ln.template fft<-1>(v);
+      if (!spectral) ln.forward(v);
       if (next_p >= 0) nx.p0 = a.passes[next_backward ? nx.st.bwd_off : nx.st.fwd_off];
       const int pid0 = (pid && own_if) ? pid[q0] : 0;
-      if (npass > 1 && own) {
+      if (npass > 1) {
 #pragma unroll
-        for (int m = 0; m < E; ++m) S[ln.pos(m)] = v[m];
+        for (int s2 = 0; s2 < S; ++s2)
+          if (ln.sown(s2)) spec_line[ln.sidx(s2)] = v[s2];
       }
       spectral = npass == 1 && !mk && !has_add && slot < 0 && s + 1 < a.nz;
       for (int j = 0; j < npass; ++j) {
         PassRec nxt = cur;
         if (j + 1 < npass) {
           nxt = a.passes[off + j + 1];
-          if (own) {
-            const C* mn = static_cast<const C*>(nxt.tab) + eoff;
+          const C* mn = static_cast<const C*>(nxt.tab) + eoff;
 #pragma unroll
-            for (int m = 0; m < E; ++m) ch::op_prefetch(mn, ln.pos(m), n);
-          }
+          for (int s2 = 0; s2 < S; ++s2)
+            if (ln.sown(s2)) ch::op_prefetch(mn, ln.spos(s2), n);
         }
         const C* tab = static_cast<const C*>(cur.tab) + eoff;
-        if (own) {
 #pragma unroll
-          for (int m = 0; m < E; ++m) {
-            const int q = ln.pos(m);
-            v[m] = ch::op(npass > 1 ? S[q] : v[m], tab, q, n);
-            if ((m & 3) == 3) asm volatile("" ::: "memory");
-          }
+        for (int s2 = 0; s2 < S; ++s2) {
+          if (ln.sown(s2)) v[s2] = ch::op(npass > 1 ? spec_line[ln.sidx(s2)] : v[s2], tab, ln.spos(s2), n);
+          if ((s2 & 3) == 3) asm volatile("" ::: "memory");
         }
         if (spectral) {  // FP32 tables carry 1/N for the inverse transform left out here
-          if (sizeof(T) != sizeof(double) && own) {
+          if constexpr (sizeof(T) != sizeof(double)) {
 #pragma unroll
-            for (int m = 0; m < E; ++m) v[m] = v[m] * static_cast<T>(n);
+            for (int s2 = 0; s2 < S; ++s2) v[s2] = v[s2] * static_cast<T>(n);
           }
           break;
         }
-        ln.template fft<+1>(v);
+        ln.inverse(v);
         if (own) {
 #pragma unroll
           for (int m = 0; m < E; ++m) v[m] = v[m] * a.inv_n;
@@ -271,24 +363,24 @@ __global__ void __launch_bounds__(Line::kMaxThreads, 1)
           if (own) {
 #pragma unroll
             for (int m = 0; m < E; ++m) {
-              const int q = ln.pos(m);
-              if (mk) v[m] = ch::masked(v[m], mk, q, n);
+              if (mk) v[m] = ch::masked(v[m], mk, a.mask_smem ? ln.lpos(m) : ln.pos(m), mo);
               if (!pid || unpack_pid<E>(pw, m) == cur.pair) out[m] = v[m];
             }
           }
         } else {  // gather at the interface pixels through the free exchange line
-          C* buf = ln.phase ? ln.b1 : ln.b0;
+          C* buf = in.phase ? in.b1 : in.b0;
           if (own) {
 #pragma unroll
-            for (int m = 0; m < E; ++m) buf[rf::pad<T>(ln.pos(m))] = v[m];
+            for (int m = 0; m < E; ++m) buf[rf::pad<T>(ln.lpos(m))] = v[m];
           }
           __syncthreads();
-          if (own_if && (!pid || pid0 == cur.pair)) store[2 * t] = buf[rf::pad<T>(q0)];
+          if (own_if && ln.mine(q0) && (!pid || pid0 == cur.pair))
+            store[2 * t] = buf[rf::pad<T>(ln.local(q0))];
           for (int k = t + nthr; k < st.niface; k += nthr) {
             const int q = iface[k];
-            if (!pid || pid[q] == cur.pair) store[2 * k] = buf[rf::pad<T>(q)];
+            if (ln.mine(q) && (!pid || pid[q] == cur.pair)) store[2 * k] = buf[rf::pad<T>(ln.local(q))];
           }
-          ln.phase ^= 1;
+          in.phase ^= 1;
         }
         cur = nxt;
       }
@@ -298,26 +390,28 @@ __global__ void __launch_bounds__(Line::kMaxThreads, 1)
         for (int m = 0; m < E; ++m) v[m] = out[m];
       }
       if (has_add) {  // sparse sources at this step's interface pixels
-        C* buf = ln.phase ? ln.b1 : ln.b0;
+        C* buf = in.phase ? in.b1 : in.b0;
         if (own) {
 #pragma unroll
-          for (int m = 0; m < E; ++m) buf[rf::pad<T>(ln.pos(m))] = v[m];
+          for (int m = 0; m < E; ++m) buf[rf::pad<T>(ln.lpos(m))] = v[m];
         }
         __syncthreads();
-        if (own_if) {
-          const int q = rf::pad<T>(q0);
+        if (own_if && ln.mine(q0)) {
+          const int q = rf::pad<T>(ln.local(q0));
           buf[q] = buf[q] + a0;
         }
         for (int k = t + nthr; k < st.niface; k += nthr) {
-          const int q = rf::pad<T>(iface[k]);
+          const int g = iface[k];
+          if (!ln.mine(g)) continue;
+          const int q = rf::pad<T>(ln.local(g));
           buf[q] = buf[q] + add[2 * k];
         }
         __syncthreads();
         if (own) {
 #pragma unroll
-          for (int m = 0; m < E; ++m) v[m] = buf[rf::pad<T>(ln.pos(m))];
+          for (int m = 0; m < E; ++m) v[m] = buf[rf::pad<T>(ln.lpos(m))];
         }
-        ln.phase ^= 1;
+        in.phase ^= 1;
       }
       if (slot >= 0 && own) {
 #pragma unroll
@@ -331,6 +425,7 @@ __global__ void __launch_bounds__(Line::kMaxThreads, 1)
       for (int m = 0; m < E; ++m) dst[2 * ln.pos(m)] = v[m];
     }
   }
+  if constexpr (K > 1) cl::cg::this_cluster().sync();  // no CTA leaves while a peer may still send
 }
 
 // ---- host side ---------------------------------------------------------------------------------
@@ -342,10 +437,13 @@ __global__ void __launch_bounds__(Line::kMaxThreads, 1)
 template <typename T>
 inline void chain_smem(int n, bool masked, ChainKernel& k) {
   const std::size_t cap = 220 * 1024;
-  const std::size_t line = static_cast<std::size_t>(rf::padded<T>(n)) * sizeof(cx<T>);
-  const std::size_t mask = (8 * static_cast<std::size_t>(n) + 15) / 16 * 16;
-  const std::size_t tw = static_cast<std::size_t>(n - 1) * sizeof(Tw<T>);
+  const int m = n / k.ctas, mb = (m + k.ctas - 1) / k.ctas;
+  const std::size_t line = static_cast<std::size_t>(rf::padded<T>(m)) * sizeof(cx<T>);
+  const std::size_t mask = (8 * static_cast<std::size_t>(m) + 15) / 16 * 16;
+  const std::size_t tw = static_cast<std::size_t>(m - 1) * sizeof(Tw<T>);
+  const std::size_t spec = static_cast<std::size_t>(k.ctas) * mb * sizeof(cx<T>);
   k.smem = 2 * line;
+  if (k.ctas > 1) k.smem += 2 * spec + (m + static_cast<std::size_t>(k.ctas) * mb) * sizeof(Tw<T>);
   if (k.smem > cap) {
     k.fn = nullptr;
     return;
@@ -354,55 +452,70 @@ inline void chain_smem(int n, bool masked, ChainKernel& k) {
   if (k.tw_smem) k.smem += tw;
   k.mask_smem = masked && k.smem + mask <= cap;
   if (k.mask_smem) k.smem += mask;
-  k.spec_smem = k.smem + n * sizeof(cx<T>) <= cap;
-  if (k.spec_smem) k.smem += n * sizeof(cx<T>);
+  k.spec_smem = k.smem + spec <= cap;
+  if (k.spec_smem) k.smem += spec;
 }
 
-template <typename T, int N, int NT, int... R>
+// Compiled lengths: K parts of N points on NT threads each.
+template <typename T, int K, int N, int NT, int... R>
 inline ChainKernel chain_fixed() {
+  using In = ch::FixedLine<T, N, NT, rf::Radices<R...>>;
   ChainKernel k;
-  k.fn = (const void*)k_chain2d<ch::FixedLine<T, N, NT, rf::Radices<R...>>>;
+  if constexpr (K == 1)
+    k.fn = (const void*)k_chain2d<ch::Whole<In>>;
+  else
+    k.fn = (const void*)k_chain2d<ch::Split<In, K>>;
+  k.ctas = K;
   k.threads = NT;
   k.radices = {R...};
   return k;
 }
 
-// Run-time lengths: the kernel of E values per thread and its thread limit.
+// Run-time lengths from here on are split over a cluster where they divide (FP64, µs per step, whole →
+// split: 1000 points 4.9 → 4.7, 1080 6.1 → 4.6, 1500 7.1 → 5.3; complex64 5.2 → 5.4, 6.1 → 4.8,
+// 7.3 → 5.8; 900 points and below gain nothing).
+constexpr int kChainSplitMin = 1024;
+
+// Run-time lengths: the kernel of E values per thread, its thread limit and parts per line.
 struct ChainRuntime {
-  int e, max_threads;
+  int e, max_threads, ctas;
   const void* fn;
 };
 template <typename T, int E>
 inline void chain_runtime(std::vector<ChainRuntime>& v) {
-  v.push_back({E, 256, (const void*)k_chain2d<ch::RuntimeLine<T, E, 256>>});
-  v.push_back({E, 384, (const void*)k_chain2d<ch::RuntimeLine<T, E, 384>>});
-  v.push_back({E, 512, (const void*)k_chain2d<ch::RuntimeLine<T, E, 512>>});
+  v.push_back({E, 256, 1, (const void*)k_chain2d<ch::Whole<ch::RuntimeLine<T, E, 256>>>});
+  v.push_back({E, 384, 1, (const void*)k_chain2d<ch::Whole<ch::RuntimeLine<T, E, 384>>>});
+  v.push_back({E, 512, 1, (const void*)k_chain2d<ch::Whole<ch::RuntimeLine<T, E, 512>>>});
+}
+template <typename T, int E, int K>
+inline void chain_runtime_split(std::vector<ChainRuntime>& v) {
+  v.push_back({E, 256, K, (const void*)k_chain2d<ch::Split<ch::RuntimeLine<T, E, 256>, K>>});
 }
 
-// The run-time kernel of length n: the E (E² divides n, n/E within the thread limit) with the
-// smallest estimate, in the form with the most registers that takes n/E threads (at 128 registers
-// FP64 lines spill: 2430 points 17.0 µs per step, 13.7 at 168). 900 FP64 points: E = 5 5.6 µs,
-// 3 5.8, 2 6.5, 6 6.9, 10 10.6. Lengths without such an E keep the launch-per-step kernels.
-inline ChainKernel chain_pick_runtime(const std::vector<ChainRuntime>& all, int n) {
+// The run-time kernel of length n among those of `ctas` parts: the E (E² divides n/ctas, within the
+// thread limit) with the smallest cost, in the form with the most registers that takes its threads
+// (at 128 registers FP64 lines spill: 2430 points 17.0 µs per step, 13.7 at 168). 900 FP64 points:
+// E = 5 5.6 µs, 3 5.8, 2 6.5, 6 6.9, 10 10.6. Lengths without such an E keep the launch-per-step
+// kernels.
+inline ChainKernel chain_pick_runtime(const std::vector<ChainRuntime>& all, int n, int ctas) {
   ChainKernel best;
-  double best_score = 1e30;
+  double best_score = 1e29;
   int best_e = 0;
-  const char* force = std::getenv("BWPM_CHAIN_E");  // tuning measurements
+  if (n % ctas || n >= 1 << 15) return best;
+  const int m = n / ctas;
   for (const ChainRuntime& c : all) {
-    if (force && std::atoi(force) != c.e) continue;
     // ordered by thread limit: the first that takes n has the most registers
-    if (c.e == best_e || n % (c.e * c.e) || n / c.e > c.max_threads || n >= 1 << 15) continue;
-    const int threads = (n / c.e + 31) / 32 * 32;
-    std::vector<int> inner;
-    const double score = 2 * (14.0 + c.e) + chain_inner(n / (c.e * c.e), n, threads, 10, inner);
+    if (c.ctas != ctas || c.e == best_e || m % c.e || m / c.e > c.max_threads) continue;
+    const int threads = (m / c.e + 31) / 32 * 32;
+    std::vector<int> radices;
+    const double score = equal_outer_plan(m, c.e, threads, radices);
     if (score < best_score - 1e-9) {
       best_score = score;
       best_e = c.e;
       best.fn = c.fn;
+      best.ctas = ctas;
       best.threads = threads;
-      best.radices = {c.e};
-      best.radices.insert(best.radices.end(), inner.begin(), inner.end());
-      best.radices.push_back(c.e);
+      best.radices = radices;
     }
   }
   return best;

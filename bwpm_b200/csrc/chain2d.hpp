@@ -11,9 +11,10 @@ namespace bwpm {
 
 struct ChainKernel {
   const void* fn = nullptr;   // null: no chain kernel for the length (or its shared memory)
+  int ctas = 1;               // CTAs per line (a cluster when more than one)
   int threads = 0;
   std::size_t smem = 0;       // dynamic shared memory per CTA
-  std::vector<int> radices;   // the transform's stages
+  std::vector<int> radices;   // of the n / ctas points of a part
   int tw_smem = 0;            // the stage twiddles sit in shared memory
   int mask_smem = 0;          // the mask does
   int spec_smem = 0;          // the spectrum line of a multi-pass step does

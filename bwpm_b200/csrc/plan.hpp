@@ -97,9 +97,13 @@ inline HostPlan make_plan_radices(int n, const std::vector<int>& radices) {
   return hp;
 }
 
-// Plan (E, inner radices, E) of length n: the inner radices (10 to 2) with the smallest estimate
-// over their stages for nt threads; empty when E² does not divide n or a prime above 7 is left.
-// A stage costs about 6 value-times of latency per round of butterflies beside its values.
+// Cost of a stage of radix r in `rounds` rounds of butterflies, in value-times of a thread: mostly
+// its serial butterfly (fitted to run-time-length kernels of 900-1000 points: complex64 1000 points
+// E = 5 on 200 threads 4.7 µs per step, E = 10 on 100 threads 7.1).
+inline double stage_cost(int r, double rounds) { return 4.0 + rounds * (1.0 + 1.5 * r); }
+
+// Plan (E, inner radices, E) of length n: the inner radices (10 to 2, product m) with the smallest
+// cost for nthr threads in `out`; returns their cost, 1e30 when a prime above 7 is left.
 inline double chain_inner(int m, int n, int nthr, int max_radix, std::vector<int>& out) {
   if (m == 1) return 0.0;
   double best = 1e30;
@@ -107,9 +111,7 @@ inline double chain_inner(int m, int n, int nthr, int max_radix, std::vector<int
   for (int r = std::min(max_radix, 10); r >= 2; --r) {
     if (m % r) continue;
     std::vector<int> rest;
-    const double tail = chain_inner(m / r, n, nthr, r, rest);
-    const double rounds = (n / r + nthr - 1) / nthr;
-    const double cost = tail + 8.0 + rounds * (6.0 + r);
+    const double cost = chain_inner(m / r, n, nthr, r, rest) + stage_cost(r, (n / r + nthr - 1) / nthr);
     if (cost < best - 1e-9) {
       best = cost;
       pick = {r};
@@ -118,6 +120,19 @@ inline double chain_inner(int m, int n, int nthr, int max_radix, std::vector<int
   }
   out = pick;
   return best;
+}
+
+// Cost of the whole plan, its radices in `radices`.
+inline double equal_outer_plan(int n, int e, int nthr, std::vector<int>& radices) {
+  radices.clear();
+  if (n % (e * e)) return 1e30;
+  std::vector<int> inner;
+  const double cost = 2 * stage_cost(e, 1.0) + chain_inner(n / (e * e), n, nthr, 10, inner);
+  if (cost >= 1e29) return 1e30;
+  radices.push_back(e);
+  radices.insert(radices.end(), inner.begin(), inner.end());
+  radices.push_back(e);
+  return cost;
 }
 
 // Threads needed so that every stage fits its register staging of EPT values per thread

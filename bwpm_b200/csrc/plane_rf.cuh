@@ -589,17 +589,17 @@ inline RfRuntime<T> rf_runtime() {
 }
 
 // The run-time kernels of length n: the E (E² divides n, n/E threads per component and line) with
-// the smallest estimate (chain_inner), two lines per CTA where they fit. Lengths without such an E
+// the smallest cost (equal_outer_plan), two lines per CTA where they fit. Lengths without such an E
 // keep the general kernels.
 template <typename T>
 inline RfKernels rf_pick_runtime(const std::vector<RfRuntime<T>>& all, int n) {
   RfKernels best;
-  double best_score = 1e30;
+  double best_score = 1e29;
   for (const RfRuntime<T>& c : all) {
-    if (n % (c.e * c.e) || 2 * (n / c.e) > kRfThreads || n >= 1 << 15 || rf_smem<T>(n, 1, true) > 200 * 1024) continue;
+    if (2 * (n / c.e) > kRfThreads || n >= 1 << 15 || rf_smem<T>(n, 1, true) > 200 * 1024) continue;
     const int nt = n / c.e;
-    std::vector<int> inner;
-    const double score = 2 * (14.0 + c.e) + chain_inner(n / (c.e * c.e), n, nt, 10, inner);
+    std::vector<int> radices;
+    const double score = equal_outer_plan(n, c.e, nt, radices);
     if (score >= best_score - 1e-9) continue;
     best_score = score;
     best.cols = c.cols;
@@ -609,9 +609,7 @@ inline RfKernels rf_pick_runtime(const std::vector<RfRuntime<T>>& all, int n) {
     best.threads = (2 * best.lines * nt + 31) / 32 * 32;
     best.cols_smem = rf_smem<T>(n, best.lines, true);
     best.rows_smem = rf_smem<T>(n, best.lines, false);
-    best.radices = {c.e};
-    best.radices.insert(best.radices.end(), inner.begin(), inner.end());
-    best.radices.push_back(c.e);
+    best.radices = radices;
   }
   return best;
 }

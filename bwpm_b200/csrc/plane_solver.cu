@@ -124,6 +124,23 @@ class PlaneSolver final : public Solver {
     ++launches_;
   }
 
+  // `grid` CTAs in clusters of `ctas`
+  void launch_cluster(const void* fn, int grid, int ctas, int threads, std::size_t smem, void** args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(ctas);
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(grid));
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream_;
+    cfg.attrs = attr;
+    cfg.numAttrs = ctas > 1 ? 1 : 0;
+    check_cuda(cudaLaunchKernelExC(&cfg, fn, args), "kernel launch");
+    ++launches_;
+  }
+
   // a register-resident 3D kernel, its prologue overlapping the end of the kernel before
   // (programmatic dependent launch)
   template <class A>
@@ -192,6 +209,7 @@ class PlaneSolver final : public Solver {
   HostPlan chain_plan_;
   DevBuf<Tw<T>> tw_chain_;
   DevBuf<R2Step> chain_steps_;
+  DevBuf<C> chain_spec_;
   int sms_ = 148;
   LaunchShape rows2_, rows3_, sel_, cols1_, cols2_, cols3_;
   std::int64_t launches_ = 0, gmres_applies_ = 0;
@@ -209,6 +227,22 @@ class PlaneSolver final : public Solver {
   std::vector<int> pass_nt_[2], pass_nr_[2];
   int pool_dirs_ = 0;  // directions in the pool: 0 none, 1 forward, 2 forward and backward
 };
+
+// A part's plan (m points) with its m − 1 stage twiddles followed, for lines split over several CTAs,
+// by the cross twiddles w_N^{c·k} (c < ctas, k < m), N = ctas·m.
+inline HostPlan with_cross_twiddles(HostPlan plan, int ctas) {
+  const long long m = plan.plan.n, n = m * ctas;
+  plan.twiddles.resize(static_cast<std::size_t>(m - 1));
+  if (ctas > 1)
+    for (long long c = 0; c < ctas; ++c)
+      for (long long k = 0; k < m; ++k) {
+        const double ang = -6.283185307179586476925286766559 * static_cast<double>((c * k) % n) /
+                           static_cast<double>(n);
+        plan.twiddles.push_back(cd{std::cos(ang), std::sin(ang)});
+      }
+  if (plan.twiddles.empty()) plan.twiddles.push_back(cd{1.0, 0.0});
+  return plan;
+}
 
 template <typename T>
 LaunchShape PlaneSolver<T>::rows_shape(int ncomp, int rows_max) const {
@@ -531,8 +565,15 @@ void PlaneSolver<T>::setup() {
     if (hosts_.empty() && in_.nz > 0 && !(k2 && std::strcmp(k2, "step") == 0))
       chain_ = chain_kernel<T>(static_cast<int>(in_.ny), !in_.mask.empty());
     if (chain_.fn) {
-      chain_plan_ = make_plan_radices(static_cast<int>(in_.ny), chain_.radices);
-      upload_tw(chain_plan_, tw_chain_);
+      chain_plan_ = make_plan_radices(static_cast<int>(in_.ny) / chain_.ctas, chain_.radices);
+      upload_tw(with_cross_twiddles(chain_plan_, chain_.ctas), tw_chain_);
+      if (!chain_.spec_smem) {  // every part's block
+        const int m = static_cast<int>(in_.ny) / chain_.ctas;
+        chain_spec_.alloc(2 * static_cast<std::size_t>(chain_.ctas) * chain_.ctas *
+                              ((m + chain_.ctas - 1) / chain_.ctas), stream_);
+      }
+      status_.alloc(1, stream_);
+      check_cuda(cudaMemsetAsync(status_.ptr, 0, sizeof(int), stream_), "memset");
       check_cuda(cudaFuncSetAttribute(chain_.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(chain_.smem)), "smem");
     }
@@ -627,18 +668,7 @@ void PlaneSolver<T>::setup() {
     if (born_k_.fn) {
       const int m = static_cast<int>(in_.ny) / born_k_.ctas;
       born_plan_ = make_plan_radices(m, born_k_.radices);
-      HostPlan all = born_plan_;  // stage twiddles, then w_N^{c·k}
-      all.twiddles.resize(static_cast<std::size_t>(m - 1));
-      if (born_k_.ctas > 1)
-        for (int c = 0; c < born_k_.ctas; ++c)
-          for (int k = 0; k < m; ++k) {
-            const double ang = -6.283185307179586476925286766559 *
-                               static_cast<double>((static_cast<long long>(c) * k) % static_cast<long long>(in_.ny)) /
-                               static_cast<double>(in_.ny);
-            all.twiddles.push_back(cd{std::cos(ang), std::sin(ang)});
-          }
-      if (all.twiddles.empty()) all.twiddles.push_back(cd{1.0, 0.0});
-      upload_tw(all, tw_born_);
+      upload_tw(with_cross_twiddles(born_plan_, born_k_.ctas), tw_born_);
       for (std::size_t i = 0; i < hosts_.size(); ++i) {
         DevBuf<cd>& d = born_modes_[{hosts_[i].re, hosts_[i].im}];
         if (d.n) continue;
@@ -859,20 +889,18 @@ void PlaneSolver<T>::chain(int iterations, const std::vector<int>& keep_slot, bo
   a.src_fwd = src_fwd_.ptr;
   a.src_bwd = src_bwd_.ptr;
   a.mask = mask_.ptr;
-  a.spec = spec_.ptr;
+  a.spec = chain_spec_.ptr;
   a.tw = tw_chain_.ptr;
   a.n = static_cast<int>(n());
   a.nz = static_cast<int>(in_.nz);
   a.iterations = iterations;
-  a.ntw = static_cast<int>(n()) - 1;
+  a.status = status_.ptr;
   a.tw_smem = chain_.tw_smem;
   a.mask_smem = chain_.mask_smem;
   a.spec_smem = chain_.spec_smem;
   a.inv_n = sizeof(T) == sizeof(double) ? static_cast<T>(1.0 / static_cast<double>(n())) : T(1);
   void* args[] = {&a, &chain_plan_.plan};
-  check_cuda(cudaLaunchKernel(chain_.fn, dim3(2), dim3(chain_.threads), args, chain_.smem, stream_),
-             "k_chain2d");
-  ++launches_;
+  launch_cluster(chain_.fn, 2 * chain_.ctas, chain_.ctas, chain_.threads, chain_.smem, args);
   last_e_ = e_.ptr;
 }
 
@@ -1309,20 +1337,8 @@ void PlaneSolver<T>::born_slab(int slot, int dir, const C* in, const C* step_tab
   a.dir = dir;
   a.basis_smem = born_k_.basis_smem;
   a.tol = in_.gmres_tol;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(born_k_.ctas);
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(born_k_.ctas);
-  cfg.blockDim = dim3(born_k_.threads);
-  cfg.dynamicSmemBytes = born_k_.smem;
-  cfg.stream = stream_;
-  cfg.attrs = attr;
-  cfg.numAttrs = born_k_.ctas > 1 ? 1 : 0;
   void* args[] = {&a, &born_plan_.plan};
-  check_cuda(cudaLaunchKernelExC(&cfg, born_k_.fn, args), "k_born2d");
-  ++launches_;
+  launch_cluster(born_k_.fn, born_k_.ctas, born_k_.ctas, born_k_.threads, born_k_.smem, args);
   born_graph_used_ = true;  // its error flag and counts are read at the end of the run
 }
 
@@ -1563,7 +1579,7 @@ void PlaneSolver<T>::run(const cd* field, int iterations, const std::int64_t* ke
     check_cuda(cudaMemcpy(&st, status_.ptr, sizeof(int), cudaMemcpyDeviceToHost), "status");
     if (st) {
       check_cuda(cudaMemsetAsync(status_.ptr, 0, sizeof(int), stream_), "status");
-      throw std::runtime_error(is2d() ? "an exchange of the Born slab did not complete in time"
+      throw std::runtime_error(is2d() ? "an exchange of a split 2D line did not complete in time"
                                       : "a bulk copy of the 3D slab step did not complete in time");
     }
   }

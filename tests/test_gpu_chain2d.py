@@ -1,7 +1,7 @@
 """The 2D chain kernels (bwpm_b200/csrc/chain2d.cuh) on a GPU.
 
-Every sweep of a 2D solve runs in one launch, with compiled lengths (256 … 4096) and run-time
-ones (n = E²·m). A volume with three materials (one absorbing), a tilted face, so steps of one
+Every sweep of a 2D solve runs in one launch, with compiled lengths (256 … 8192) and run-time
+ones, on one CTA or split over a cluster. A volume with three materials (one absorbing), a tilted face, so steps of one
 and of several passes, and a planar end goes through the chain kernels and through the
 launch-per-step kernels (BWPM_2D_KERNELS=step), and both are held to the numpy oracle: FP64 at
 the drop-in contract (1e-10), complex64 at the complex64 contract (relative L2 ≤ 1e-4). Without a
@@ -41,8 +41,8 @@ def _case(ny: int, nz: int, masked: bool):
 
 
 @pytest.mark.parametrize("masked", [True, False])
-@pytest.mark.parametrize("ny", [4, 18, 150, 210, 256, 343, 375, 384, 512, 768, 1024, 1080, 1536,
-                                2048, 2187, 3072, 3600, 4050, 4096, 5120, 6144, 8192])
+@pytest.mark.parametrize("ny", [4, 18, 150, 210, 256, 343, 375, 384, 512, 768, 1024, 1080, 1500, 1536, 1944,
+                                2048, 2187, 2430, 2500, 3072, 3600, 4050, 4096, 5120, 6144, 8192])
 def test_chain_matches_step_kernels_and_oracle(monkeypatch, ny, masked):
     from bwpm_b200 import _core
     from oracle import port
