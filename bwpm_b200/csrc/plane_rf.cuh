@@ -445,6 +445,7 @@ __global__ void __launch_bounds__(Line::kThreads, rfp::blocks(Line::kThreads))
   using T = typename Line::T;
   using C = cx<T>;
   constexpr int E = Line::E, EW = (E + 3) / 4;
+  __shared__ int s_pass[kMaxPasses];
   extern __shared__ __align__(16) unsigned char smem_tw[];
   const int ny = a.ny, nx = plan.n;
   unsigned char* smem_raw = smem_tw + nx * sizeof(Tw<T>);
@@ -479,26 +480,44 @@ __global__ void __launch_bounds__(Line::kThreads, rfp::blocks(Line::kThreads))
       prefetch_l1(a.mask + row + ln.pos(m));
       if constexpr (sizeof(T) != sizeof(double)) prefetch_l1(a.mask + n + row + ln.pos(m));
     }
+  // the passes of this CTA's rows: pair, and bit 16 for a reflection; −1: left out
+  for (int j = threadIdx.x; j < npass; j += blockDim.x) {
+    const PassRec r = ps[j];
+    s_pass[j] = (here >> r.pair) & 1 ? r.pair | r.refl << 16 : -1;
+  }
   __syncthreads();
   rfp::wait_previous();
-  C o[E];
+  auto next_pass = [&](int j) {
+    while (j < npass && s_pass[j] < 0) ++j;
+    return j;
+  };
+  C o[E], w[E];
 #pragma unroll
   for (int m = 0; m < E; ++m) o[m] = C{0, 0};
-  for (int j = 0; j < npass; ++j) {
-    const PassRec pr = ps[j];
-    if (!((here >> pr.pair) & 1)) continue;
+  auto load = [&](C(&v)[E], int j) {
     const C* src = a.work + static_cast<long long>(j) * 2 * n;
-    C w[E];
     if (own) {
 #pragma unroll
-      for (int m = 0; m < E; ++m) w[m] = src[(static_cast<long long>(ln.pos(m)) * ny + y) * 2 + c];
+      for (int m = 0; m < E; ++m) v[m] = src[(static_cast<long long>(ln.pos(m)) * ny + y) * 2 + c];
+    }
+  };
+  // the next pass's values load during the transform where the registers allow
+  constexpr bool kAhead = E * sizeof(C) <= 64;
+  int j = next_pass(0), jn = j;
+  if (j < npass) load(w, j);
+  for (; j < npass; j = jn) {
+    const int pair = s_pass[j] & 0xffff, refl = s_pass[j] >> 16;
+    jn = next_pass(j + 1);
+    C wn[kAhead ? E : 1];
+    if constexpr (kAhead) {
+      if (jn < npass) load(wn, jn);
     }
     ln.template fft<+1>(w);
-    if (!pr.refl) {
+    if (!refl) {
       if (own) {
 #pragma unroll
         for (int m = 0; m < E; ++m)
-          if (!a.pid || unpack_pid<E>(pw, m) == pr.pair) o[m] = w[m] * a.inv_n;
+          if (!a.pid || unpack_pid<E>(pw, m) == pair) o[m] = w[m] * a.inv_n;
       }
     } else {
       // the gather reads other threads' values: through the free buffers, natural order
@@ -510,12 +529,18 @@ __global__ void __launch_bounds__(Line::kThreads, rfp::blocks(Line::kThreads))
       __syncthreads();
       for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
         const int q = a.iface[k];
-        if (a.pid && a.pid[q] != pr.pair) continue;
+        if (a.pid && a.pid[q] != pair) continue;
         const int qy = q / nx, qx = q - qy * nx;
         const C* f = ln.free_of(smem_raw, qy - y0);
         st_px(a.refl_out + 2 * k, f[rfp::at(qx, 0)] * a.inv_n, f[rfp::at(qx, 1)] * a.inv_n);
       }
       __syncthreads();  // the next transform writes these buffers first
+    }
+    if constexpr (kAhead) {
+#pragma unroll
+      for (int m = 0; m < E; ++m) w[m] = wn[m];
+    } else {
+      if (jn < npass) load(w, jn);
     }
   }
   if (a.mask && own)
