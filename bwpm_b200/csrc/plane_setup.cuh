@@ -6,7 +6,7 @@
 // std::set order, the I_r,s selection, reflection sources where ñ(plane p) ≠ ñ(plane p + 1)),
 // done once per solve for all steps at once instead of per slab on the host: codes
 // (r + 1)·m + s sort like the pairs, a presence bitmask per step gives the pairs in order, and
-// one CTA per step compacts the interface pixels in pixel order with ballot/popc scans.
+// the interface pixels are compacted in pixel order by segment (count, scan, ballots).
 #pragma once
 
 #include <cstdint>
@@ -69,48 +69,79 @@ __global__ void k_setup_pid(SetupVolume v, const int* steps, const long long* pi
     out[q] = table[setup_code(v, p, q)];
 }
 
-// one CTA per listed step: its interface pixels in increasing pixel order at iface_off[k], and
-// (3D, rowoff_off[k] ≥ 0) the offset of each row's first entry, ny + 1 values.
+// The interface pixels of the listed steps in increasing pixel order, in three kernels over segments
+// of `seg` pixels (3D: rows): count, scan, write. (One CTA per step, scanning row by row, took
+// 0.6 ms for 12 slabs of 512² and 1.1 ms for 1024²: a dozen SMs, three barriers per row.)
+// grid (⌈nseg/8⌉, steps), one warp per segment: its number of interface pixels.
+__global__ void __launch_bounds__(256)
+    k_setup_iface_count(SetupVolume v, const int* steps, const std::uint8_t* code_iface, int seg, int nseg,
+                        int* segoff) {
+  const int s = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (s >= nseg) return;
+  const int p = steps[blockIdx.y];
+  const long long q0 = static_cast<long long>(s) * seg, q1 = min(q0 + seg, v.nn);
+  int n = 0;
+  for (long long q = q0 + lane; q < q1; q += 32) n += code_iface[setup_code(v, p, q)] != 0;
+  for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+  if (lane == 0) segoff[static_cast<long long>(blockIdx.y) * (nseg + 1) + s] = n;
+}
+
+// One CTA per step: counts → offsets (nseg + 1 values), copied to the row offsets in 3D
+// (rowoff_off[k] ≥ 0).
 __global__ void __launch_bounds__(kSetupThreads)
-    k_setup_iface(SetupVolume v, const int* steps, const long long* iface_off,
-                  const long long* rowoff_off, const std::uint8_t* code_iface, int* iface_pool,
-                  int* rowoff_pool) {
+    k_setup_iface_scan(int nseg, int* segoff, const long long* rowoff_off, int* rowoff_pool) {
   __shared__ int s_warp[kSetupThreads / 32];
-  __shared__ int s_total;
-  const int k = blockIdx.x;
-  const int p = steps[k];
-  int* out = iface_pool + iface_off[k];
+  const int k = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int* off = segoff + static_cast<long long>(k) * (nseg + 1);
   int* rowoff = rowoff_off[k] >= 0 ? rowoff_pool + rowoff_off[k] : nullptr;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int running = 0;  // entries written so far (uniform across the CTA)
-  const int row_len = rowoff ? v.nx : static_cast<int>(v.nn < (1LL << 30) ? v.nn : (1LL << 30));
-  const int rows = rowoff ? v.ny : 1;
-  for (int y = 0; y < rows; ++y) {
-    if (rowoff && threadIdx.x == 0) rowoff[y] = running;
-    const long long base = rowoff ? static_cast<long long>(y) * v.nx : 0;
-    for (int c0 = 0; c0 < row_len; c0 += kSetupThreads) {
-      const int x = c0 + threadIdx.x;
-      const long long q = base + x;
-      const bool flag = x < row_len && code_iface[setup_code(v, p, q)];
-      const unsigned ballot = __ballot_sync(0xffffffffu, flag);
-      if (lane == 0) s_warp[warp] = __popc(ballot);
-      __syncthreads();
-      if (threadIdx.x == 0) {  // exclusive scan of the warp counts
-        int acc = 0;
-        for (int w = 0; w < kSetupThreads / 32; ++w) {
-          const int c = s_warp[w];
-          s_warp[w] = acc;
-          acc += c;
-        }
-        s_total = acc;
-      }
-      __syncthreads();
-      if (flag) out[running + s_warp[warp] + __popc(ballot & ((1u << lane) - 1u))] = static_cast<int>(q);
-      running += s_total;
-      __syncthreads();
+  int running = 0;  // uniform across the CTA
+  for (int base = 0; base < nseg; base += kSetupThreads) {
+    const int i = base + threadIdx.x;
+    const int c = i < nseg ? off[i] : 0;
+    int sum = c;  // inclusive scan of the warp
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += up;
     }
+    if (lane == 31) s_warp[warp] = sum;
+    __syncthreads();
+    int before = running, total = 0;
+    for (int w = 0; w < kSetupThreads / 32; ++w) {
+      if (w < warp) before += s_warp[w];
+      total += s_warp[w];
+    }
+    if (i < nseg) {
+      off[i] = before + sum - c;
+      if (rowoff) rowoff[i] = before + sum - c;
+    }
+    running += total;
+    __syncthreads();
   }
-  if (rowoff && threadIdx.x == 0) rowoff[rows] = running;
+  if (threadIdx.x == 0) {
+    off[nseg] = running;
+    if (rowoff) rowoff[nseg] = running;
+  }
+}
+
+// grid as k_setup_iface_count: the pixels of each segment at its offset.
+__global__ void __launch_bounds__(256)
+    k_setup_iface_write(SetupVolume v, const int* steps, const long long* iface_off,
+                        const std::uint8_t* code_iface, int seg, int nseg, const int* segoff,
+                        int* iface_pool) {
+  const int s = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (s >= nseg) return;
+  const int k = blockIdx.y, p = steps[k];
+  const int* off = segoff + static_cast<long long>(k) * (nseg + 1) + s;
+  if (off[0] == off[1]) return;
+  int* out = iface_pool + iface_off[k] + off[0];
+  const long long q0 = static_cast<long long>(s) * seg, q1 = min(q0 + seg, v.nn);
+  for (long long b = q0; b < q1; b += 32) {
+    const long long q = b + lane;
+    const bool flag = q < q1 && code_iface[setup_code(v, p, q)];
+    const unsigned ballot = __ballot_sync(0xffffffffu, flag);
+    if (flag) out[__popc(ballot & ((1u << lane) - 1u))] = static_cast<int>(q);
+    out += __popc(ballot);
+  }
 }
 
 // One warp per row of the pair-id planes: bit i of row_pairs[row] when pair i occurs in it (a step

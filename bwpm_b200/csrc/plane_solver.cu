@@ -792,9 +792,19 @@ void PlaneSolver<T>::device_steps(const std::uint8_t* labels_u8, const std::vect
     d_steps.upload(with_iface.data(), with_iface.size());
     d_ioff.upload(iface_off.data(), iface_off.size());
     d_roff.upload(rowoff_off.data(), rowoff_off.size());
-    k_setup_iface<<<static_cast<unsigned>(with_iface.size()), kSetupThreads, 0, stream_>>>(
-        v, d_steps.ptr, d_ioff.ptr, d_roff.ptr, d_iface.ptr, iface_pool_.ptr, rowoff_pool_.ptr);
-    check_cuda(cudaGetLastError(), "k_setup_iface");
+    // per segment (3D: a row) the count, its scan per step, then the pixels
+    const int seg = is2d() ? 1024 : static_cast<int>(in_.nx);
+    const int nseg = static_cast<int>(ceil_div(nn, static_cast<std::size_t>(seg)));
+    const unsigned nsteps = static_cast<unsigned>(with_iface.size());
+    DevBuf<int> segoff(static_cast<std::size_t>(nsteps) * (nseg + 1), stream_);
+    const dim3 warps(ceil_div(static_cast<std::size_t>(nseg), std::size_t{8}), nsteps);
+    k_setup_iface_count<<<warps, 256, 0, stream_>>>(v, d_steps.ptr, d_iface.ptr, seg, nseg, segoff.ptr);
+    check_cuda(cudaGetLastError(), "k_setup_iface_count");
+    k_setup_iface_scan<<<nsteps, kSetupThreads, 0, stream_>>>(nseg, segoff.ptr, d_roff.ptr, rowoff_pool_.ptr);
+    check_cuda(cudaGetLastError(), "k_setup_iface_scan");
+    k_setup_iface_write<<<warps, 256, 0, stream_>>>(v, d_steps.ptr, d_ioff.ptr, d_iface.ptr, seg, nseg,
+                                                    segoff.ptr, iface_pool_.ptr);
+    check_cuda(cudaGetLastError(), "k_setup_iface_write");
     check_cuda(cudaStreamSynchronize(stream_), "setup iface");
   }
 }
