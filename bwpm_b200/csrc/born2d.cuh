@@ -4,7 +4,7 @@
 // field increment, the sources of the back-scatter and the plane they radiate. As one CUDA graph
 // per Born step (build_born_graph in plane_solver.cu, which 3D volumes and other lengths keep)
 // that is ≈ 100 small dependent kernels of 2-5 µs on a line of a few thousand points: 730 µs per
-// slab and direction at 4096 points in FP64, 118 µs here. The three components' lines are split over a
+// slab and direction at 4096 points in FP64, 106 µs here. The three components' lines are split over a
 // cluster of C CTAs and stay on chip: N = C·M, CTA c holds the real-space points C·m + c and a
 // block of the spectrum, a transform is a local register-resident M-point transform and one
 // all-to-all through distributed shared memory (the scheme of cluster2d.cuh). A thread group per
@@ -178,6 +178,9 @@ __global__ void __launch_bounds__(born_threads<Inner>(), 1)
   }
   const double inv_n = 1.0 / static_cast<double>(n);
   for (int i = tid; i < M; i += blockDim.x) pot[i] = a.pot[C * i + rank] * static_cast<T>(inv_n);
+  // constants so far; what other kernels of the run write is read after the wait (programmatic
+  // dependent launch: this prologue overlaps the slab before)
+  asm volatile("griddepcontrol.launch_dependents;");
   L ln{Inner(s_plan, s_magic, M, tws, lines + 2 * comp * pm, t, group_threads), rank, comp, M, MB, mb, xfs, xis};
   const unsigned field_bytes = static_cast<unsigned>(3 * C * mb * sizeof(V));      // forward
   const unsigned inv_bytes = static_cast<unsigned>(3 * M * sizeof(V));             // inverse
@@ -185,6 +188,7 @@ __global__ void __launch_bounds__(born_threads<Inner>(), 1)
     cl::cg::this_cluster().sync();
   else
     __syncthreads();
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const bool own = ln.own();
   const double dir = static_cast<double>(a.dir);
   auto mode = [&](int f, int s) { return modes[f * C * MB + ln.slot(s)]; };

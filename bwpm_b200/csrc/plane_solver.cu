@@ -124,19 +124,29 @@ class PlaneSolver final : public Solver {
     ++launches_;
   }
 
-  // `grid` CTAs in clusters of `ctas`
-  void launch_cluster(const void* fn, int grid, int ctas, int threads, std::size_t smem, void** args) {
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = static_cast<unsigned>(ctas);
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  // `grid` CTAs in clusters of `ctas`; programmatic: the kernel waits for its predecessor itself
+  void launch_cluster(const void* fn, int grid, int ctas, int threads, std::size_t smem, void** args,
+                      bool programmatic = false) {
+    cudaLaunchAttribute attr[2];
+    unsigned nattr = 0;
+    if (ctas > 1) {
+      attr[nattr].id = cudaLaunchAttributeClusterDimension;
+      attr[nattr].val.clusterDim.x = static_cast<unsigned>(ctas);
+      attr[nattr].val.clusterDim.y = attr[nattr].val.clusterDim.z = 1;
+      ++nattr;
+    }
+    if (programmatic) {
+      attr[nattr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[nattr].val.programmaticStreamSerializationAllowed = 1;
+      ++nattr;
+    }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(static_cast<unsigned>(grid));
     cfg.blockDim = dim3(static_cast<unsigned>(threads));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream_;
     cfg.attrs = attr;
-    cfg.numAttrs = ctas > 1 ? 1 : 0;
+    cfg.numAttrs = nattr;
     check_cuda(cudaLaunchKernelExC(&cfg, fn, args), "kernel launch");
     ++launches_;
   }
@@ -1348,7 +1358,7 @@ void PlaneSolver<T>::born_slab(int slot, int dir, const C* in, const C* step_tab
   a.basis_smem = born_k_.basis_smem;
   a.tol = in_.gmres_tol;
   void* args[] = {&a, &born_plan_.plan};
-  launch_cluster(born_k_.fn, born_k_.ctas, born_k_.ctas, born_k_.threads, born_k_.smem, args);
+  launch_cluster(born_k_.fn, born_k_.ctas, born_k_.ctas, born_k_.threads, born_k_.smem, args, true);
   born_graph_used_ = true;  // its error flag and counts are read at the end of the run
 }
 
