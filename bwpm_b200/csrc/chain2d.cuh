@@ -176,10 +176,20 @@ __device__ __forceinline__ cx<T> masked(cx<T> v, const T* m, int q, int n) {
 
 }  // namespace ch
 
-// Records of the coming step, loaded one step ahead.
-struct ChainNext {
-  R2Step st;
-  PassRec p0;
+// Step `s` of sweep `sw` in execution order, and its record's number; past the last step of the run
+// it stays where it is.
+struct ChainAt {
+  int s, sw;
+  __device__ __forceinline__ bool backward() const { return sw & 1; }
+  __device__ __forceinline__ int record(int nz) const { return backward() ? nz - 1 - s : s; }
+  __device__ __forceinline__ ChainAt next(int nz, int sweeps) const {
+    if (s + 1 < nz) return {s + 1, sw};
+    if (sw + 1 < sweeps) return {0, sw + 1};
+    return *this;
+  }
+  __device__ __forceinline__ int first_pass(const R2Step& st) const {
+    return backward() ? st.bwd_off : st.fwd_off;
+  }
 };
 
 template <class W>
@@ -270,9 +280,10 @@ __global__ void __launch_bounds__(W::In::kMaxThreads, 1)
   const int sweeps = a.iterations > 0 ? 2 * a.iterations : 1;
   const int iters = a.iterations > 0 ? a.iterations : 1;
   const int eoff = c == 0 ? 0 : 2 * n;  // m00 for E_x, m11 for E_y
-  ChainNext nx;
-  nx.st = a.steps[0];
-  nx.p0 = a.passes[nx.st.fwd_off];
+  // records ahead: the step's own, the next step's, and one pass record each
+  ChainAt at1 = ChainAt{0, 0}.next(a.nz, sweeps);
+  R2Step st0 = a.steps[0], st1 = a.steps[at1.record(a.nz)];
+  PassRec p0 = a.passes[st0.fwd_off];
   for (int sw = 0; sw < sweeps; ++sw) {
     const bool backward = sw & 1;
     const int iter = sw >> 1;
@@ -291,10 +302,13 @@ __global__ void __launch_bounds__(W::In::kMaxThreads, 1)
     bool spectral = false;  // v holds the spectrum (uniform)
     for (int s = 0; s < a.nz; ++s) {
       const int p = backward ? a.nz - 1 - s : s;  // step p: planes p and p + 1
-      const R2Step st = nx.st;
-      PassRec cur = nx.p0;
-      bool next_backward;
-      const int next_p = next_step(s, p, a.nz, sw, sweeps, backward, next_backward);
+      const R2Step st = st0;
+      PassRec cur = p0;
+      // the next step's first pass (its record is here) and the record after it: a step that stays
+      // in the spectrum is otherwise three dependent loads long
+      p0 = a.passes[at1.first_pass(st1)];
+      const ChainAt at2 = at1.next(a.nz, sweeps);
+      const R2Step st2 = a.steps[at2.record(a.nz)];
       const bool reflect = r2_reflects(st, backward, a.iterations);
       const int off = backward ? st.bwd_off : st.fwd_off;
       const int npass = r2_passes(st, backward, reflect);
@@ -303,7 +317,6 @@ __global__ void __launch_bounds__(W::In::kMaxThreads, 1)
       const C* add = (backward ? a.src_bwd : a.src_fwd) + 2 * st.iface + c;
       const std::uint8_t* pid = st.pid >= 0 ? a.pids + st.pid : nullptr;
       const int* iface = a.iface + st.iface;
-      if (next_p >= 0) nx.st = a.steps[next_p];
       const int slot = keeps ? a.keep[backward ? p : p + 1] : -1;
       // first round of the interface loops
       const bool own_if = t < st.niface;
@@ -324,7 +337,6 @@ __global__ void __launch_bounds__(W::In::kMaxThreads, 1)
           if (ln.sown(s2)) ch::op_prefetch(m0, ln.spos(s2), n);
       }
       if (!spectral) ln.forward(v);
-      if (next_p >= 0) nx.p0 = a.passes[next_backward ? nx.st.bwd_off : nx.st.fwd_off];
       const int pid0 = (pid && own_if) ? pid[q0] : 0;
       if (npass > 1) {
 #pragma unroll
@@ -384,6 +396,9 @@ __global__ void __launch_bounds__(W::In::kMaxThreads, 1)
         }
         cur = nxt;
       }
+      st0 = st1;
+      st1 = st2;
+      at1 = at2;
       if (spectral) continue;
       if (own) {
 #pragma unroll

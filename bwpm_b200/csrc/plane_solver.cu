@@ -1510,9 +1510,11 @@ void PlaneSolver<T>::run(const cd* field, int iterations, const std::int64_t* ke
     r_iter.alloc(iterations * 2 * nn, stream_);
   }
   ensure_passes(iterations > 0);
-  check_cuda(cudaMemcpyAsync(stage_.ptr, field, n2 * sizeof(cd), cudaMemcpyHostToDevice, stream_), "field upload");
-  launch(k_convert<T, double>, dim3(ceil_div(n2, kThreads)), dim3(kThreads), 0, input_.ptr,
-         (const cd*)stage_.ptr, n2);
+  void* upload_to = sizeof(T) == sizeof(double) ? static_cast<void*>(input_.ptr) : stage_.ptr;
+  check_cuda(cudaMemcpyAsync(upload_to, field, n2 * sizeof(cd), cudaMemcpyHostToDevice, stream_), "field upload");
+  if constexpr (sizeof(T) != sizeof(double))
+    launch(k_convert<T, double>, dim3(ceil_div(n2, kThreads)), dim3(kThreads), 0, input_.ptr,
+           (const cd*)stage_.ptr, n2);
   // FP64 planes are downloaded as they are, complex64 ones through a conversion
   auto download = [&](const C* src, cd* dst, cudaStream_t s) {
     if (!dst) return;
