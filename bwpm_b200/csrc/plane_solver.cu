@@ -1612,9 +1612,10 @@ std::size_t PlaneSolver<T>::device_bytes() const {
   std::size_t b = 0;
   for (auto& kv : tables_) b += kv.second.bytes();
   for (const auto* d : {&input_, &e_, &next_, &spec_, &xbuf_, &work_, &src_fwd_, &src_bwd_, &pot_,
-                        &born_fwd_, &born_bwd_, &w3_, &t3_, &sources_})
+                        &born_fwd_, &born_bwd_, &w3_, &t3_, &sources_, &born_basis_, &chain_spec_})
     b += d->bytes();
-  return b + pid_pool_.bytes() + iface_pool_.bytes() + rowoff_pool_.bytes() + mask_.bytes();
+  for (auto& kv : born_modes_) b += kv.second.bytes();
+  return b + row_pairs_.bytes() + pid_pool_.bytes() + iface_pool_.bytes() + rowoff_pool_.bytes() + mask_.bytes();
 }
 
 }  // namespace
