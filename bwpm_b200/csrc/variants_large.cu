@@ -35,7 +35,7 @@ void add_variants_large(std::vector<FixedVariant>& v) {
   v.push_back(cluster<4096, 4, 128, 8, 8, 8, 2>());
   v.push_back(cluster<4096, 8, 64, 8, 8, 8>());
   // 7.7 µs per step (8·8·8·3 9.0); two CTAs of 1536·2 points took 16.7, the same SM time
-  v.push_back(cluster<6144, 4, 192, 8, 4, 6, 8>());
+  v.push_back(cluster<6144, 4, 192, 8, 8, 3, 8>());
   v.push_back(fixed<6144, 256, 8, 8, 8, 4, 3>());
   v.push_back(cluster<6144, 8, 96, 8, 12, 8>());  // 6.5, twice the SM time
   v.push_back(cluster<8192, 4, 256, 8, 8, 8, 4>());
