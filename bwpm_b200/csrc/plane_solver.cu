@@ -52,6 +52,21 @@ struct LaunchShape {
   int group = 1;  // passes per inverse transform (row kernel of a 3D step)
 };
 
+// Raises the kernel's limit of dynamic shared memory to what the current device has beside the
+// kernel's static part. The limit belongs to the function on the device, which serves solvers of
+// many sizes at once (run-time lengths of one E, a compiled length with and without a mask, the
+// server's workers): a solver that set its own size would take the limit from one that needs more.
+// The size itself goes with each launch.
+inline void allow_smem(const void* fn) {
+  int device = 0, optin = 0;
+  check_cuda(cudaGetDevice(&device), "device");
+  check_cuda(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device), "smem");
+  cudaFuncAttributes f{};
+  check_cuda(cudaFuncGetAttributes(&f, fn), "smem");
+  check_cuda(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  optin - static_cast<int>(f.sharedSizeBytes)), "smem");
+}
+
 template <typename T>
 class PlaneSolver final : public Solver {
  public:
@@ -584,8 +599,7 @@ void PlaneSolver<T>::setup() {
       }
       status_.alloc(1, stream_);
       check_cuda(cudaMemsetAsync(status_.ptr, 0, sizeof(int), stream_), "memset");
-      check_cuda(cudaFuncSetAttribute(chain_.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(chain_.smem)), "smem");
+      allow_smem(chain_.fn);
     }
   } else {
     rows2_ = rows_shape(2, 8);
@@ -634,10 +648,8 @@ void PlaneSolver<T>::setup() {
         rf_plan_x_ = make_plan_radices(static_cast<int>(in_.nx), kx.radices);
         upload_tw(rf_plan_y_, tw_rf_y_);
         upload_tw(rf_plan_x_, tw_rf_x_);
-        check_cuda(cudaFuncSetAttribute(rf_y_.cols, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(rf_y_.cols_smem)), "smem");
-        check_cuda(cudaFuncSetAttribute(rf_x_.rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(rf_x_.rows_smem)), "smem");
+        allow_smem(rf_y_.cols);
+        allow_smem(rf_x_.rows);
         if (pid_pool_.n) {  // whole pair-id planes
           const std::size_t rows = pid_pool_.n / in_.nx;
           row_pairs_.alloc(rows, stream_);
@@ -691,8 +703,7 @@ void PlaneSolver<T>::setup() {
       check_cuda(cudaMemsetAsync(gst_.ptr, 0, sizeof(GmresState), stream_), "memset");
       status_.alloc(1, stream_);
       check_cuda(cudaMemsetAsync(status_.ptr, 0, sizeof(int), stream_), "memset");
-      check_cuda(cudaFuncSetAttribute(born_k_.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(born_k_.smem)), "smem");
+      allow_smem(born_k_.fn);
     }
   }
   check_cuda(cudaStreamSynchronize(stream_), "setup");  // this solver's stream only
