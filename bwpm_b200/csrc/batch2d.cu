@@ -109,7 +109,9 @@ int rt_choice(int n) {
     const bool outer = rv[i].equal_outer;
     const bool wide = !outer && rv[i].max_threads > rg::rt_max_threads(e);
     if (n % e || n / e > rv[i].max_threads || (wide && n / e <= rg::rt_max_threads(e))) continue;
-    if (!outer && best >= 0 && rv[best].equal_outer) break;  // listed first, and always the faster
+    // the equal-outer forms come first and their cost is another scale: where one runs n, the
+    // general forms are only taken when forced
+    if (!outer && e != forced_e && best >= 0 && rv[best].equal_outer) continue;
     const std::vector<int> r = rt_radices(n, rv[i]);
     if (r.empty()) continue;
     if (e == forced_e) return static_cast<int>(i);
