@@ -66,7 +66,7 @@ std::vector<int> rt_radices(int n, const RtVariant& rv) {
   if (rv.equal_outer) {  // (E, inner radices, E)
     for (int p : {7, 11, 13})  // 2, 3 and 5 only, as the other run-time kernels
       if (n % p == 0) return {};
-    equal_outer_plan(n, e, (n / e + 31) / 32 * 32, r);
+    equal_outer_plan(n, e, (n / e + 31) / 32 * 32, r, false);
     return r;
   }
   int m = n, twos = 0;
@@ -120,7 +120,7 @@ int rt_choice(int n) {
     double score = 0;
     if (outer) {
       std::vector<int> radices;
-      score = equal_outer_plan(n, e, (n / e + 31) / 32 * 32, radices);
+      score = equal_outer_plan(n, e, (n / e + 31) / 32 * 32, radices, false);
     } else {
       for (int x : r) score += (e % x == 0 ? 1.0 : 2.0) * (8.0 + e);
     }

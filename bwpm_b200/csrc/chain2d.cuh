@@ -507,12 +507,18 @@ inline void chain_runtime_split(std::vector<ChainRuntime>& v) {
   v.push_back({E, 256, K, (const void*)k_chain2d<ch::Split<ch::RuntimeLine<T, E, 256>, K>>});
 }
 
+// Whether E values per thread suit a line of `ctas` parts. Whole lines: 4 to 8; outer radices 2 and 3
+// cost rounding error (against the launch-per-step kernels, mean over 25 plans of E = 3: complex64 1.03,
+// FP64 1.02; E = 4 to 8 0.98, 0.90) and stages (972 points FP64 6.7 → 5.9 µs per step), above 8 a line
+// has a warp or two (225 points, E = 5 3.6 µs, 15 4.8). Parts: at most one block of the cross stage per
+// thread, E ≤ ctas (4374 points on 6 CTAs, E = 3 7.9 µs per step, E = 9 14.2).
+inline bool chain_suits(int e, int ctas) { return ctas == 1 ? e >= 4 && e <= 8 : e <= ctas; }
+
 // The run-time kernel of length n among those of `ctas` parts: the E (E² divides n/ctas, within the
 // thread limit) with the smallest cost, in the form with the most registers that takes its threads
-// (at 128 registers FP64 lines spill: 2430 points 17.0 µs per step, 13.7 at 168). 900 FP64 points:
-// E = 5 5.6 µs, 3 5.8, 2 6.5, 6 6.9, 10 10.6. Lengths without such an E keep the launch-per-step
-// kernels.
-inline ChainKernel chain_pick_runtime(const std::vector<ChainRuntime>& all, int n, int ctas) {
+// (at 128 registers FP64 lines spill: 2430 points 17.0 µs per step, 13.7 at 168). `suits`: only E that
+// suit the parts. Lengths without an E keep the launch-per-step kernels.
+inline ChainKernel chain_pick_runtime(const std::vector<ChainRuntime>& all, int n, int ctas, bool suits) {
   ChainKernel best;
   double best_score = 1e29;
   int best_e = 0;
@@ -521,6 +527,7 @@ inline ChainKernel chain_pick_runtime(const std::vector<ChainRuntime>& all, int 
   for (const ChainRuntime& c : all) {
     // ordered by thread limit: the first that takes n has the most registers
     if (c.ctas != ctas || c.e == best_e || m % c.e || m / c.e > c.max_threads) continue;
+    if (suits && !chain_suits(c.e, ctas)) continue;
     const int threads = (m / c.e + 31) / 32 * 32;
     std::vector<int> radices;
     const double score = equal_outer_plan(m, c.e, threads, radices);
@@ -534,6 +541,23 @@ inline ChainKernel chain_pick_runtime(const std::vector<ChainRuntime>& all, int 
     }
   }
   return best;
+}
+
+// The run-time chain kernel of length n, of the first part count that has a plan and its shared memory:
+// from kChainSplitMin points on those of `parts`, with an E that suits them, then with any; then the
+// whole line.
+template <typename T>
+inline ChainKernel chain_runtime_kernel(const std::vector<ChainRuntime>& all, int n, bool masked,
+                                        std::vector<int> parts) {
+  if (n < kChainSplitMin) parts.clear();
+  for (const std::vector<int>& counts : {parts, std::vector<int>{1}})
+    for (bool suits : {true, false})
+      for (int ctas : counts) {
+        ChainKernel k = chain_pick_runtime(all, n, ctas, suits);
+        if (k.fn) chain_smem<T>(n, masked, k);
+        if (k.fn) return k;
+      }
+  return ChainKernel{};
 }
 
 }  // namespace bwpm

@@ -51,13 +51,7 @@ ChainKernel chain_kernel<double>(int n, bool masked) {
         chain_runtime_split<T, 6, 8>(v);
         return v;
       }();
-      if (n >= kChainSplitMin)
-        for (int ctas : {8, 6, 5, 4}) {
-          k = chain_pick_runtime(all, n, ctas);
-          if (k.fn) chain_smem<T>(n, masked, k);
-          if (k.fn) return k;
-        }
-      k = chain_pick_runtime(all, n, 1);
+      return chain_runtime_kernel<T>(all, n, masked, {8, 6, 5, 4});
     }
   }
   if (k.fn) chain_smem<T>(n, masked, k);

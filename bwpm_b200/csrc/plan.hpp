@@ -103,7 +103,8 @@ inline HostPlan make_plan_radices(int n, const std::vector<int>& radices) {
 inline double stage_cost(int r, double rounds) { return 4.0 + rounds * (1.0 + 1.5 * r); }
 
 // Plan (E, inner radices, E) of length n: the inner radices (10 to 2, product m) with the smallest
-// cost for nthr threads in `out`; returns their cost, 1e30 when a prime above 7 is left.
+// cost for nthr threads in `out`, in decreasing order; returns their cost, 1e30 when a prime above 7 is
+// left.
 inline double chain_inner(int m, int n, int nthr, int max_radix, std::vector<int>& out) {
   if (m == 1) return 0.0;
   double best = 1e30;
@@ -122,13 +123,18 @@ inline double chain_inner(int m, int n, int nthr, int max_radix, std::vector<int
   return best;
 }
 
-// Cost of the whole plan, its radices in `radices`.
-inline double equal_outer_plan(int n, int e, int nthr, std::vector<int>& radices) {
+// Cost of the whole plan, its radices in `radices`. Chain, Born and 3D kernels take the inner radices in
+// increasing order: its rounding error, geometric mean over 126 pairs of plans of 128-6000 points on
+// facet and lens volumes, is 0.994 ± 0.002 of the decreasing order's in complex64, 0.973 ± 0.008 in FP64
+// (0.7-0.8 at 2250 and 3000 points), at 0.5 % less time. The batched engine's orders do not differ
+// (1.00 ± 0.003 over 19 lengths).
+inline double equal_outer_plan(int n, int e, int nthr, std::vector<int>& radices, bool increasing = true) {
   radices.clear();
   if (n % (e * e)) return 1e30;
   std::vector<int> inner;
   const double cost = 2 * stage_cost(e, 1.0) + chain_inner(n / (e * e), n, nthr, 10, inner);
   if (cost >= 1e29) return 1e30;
+  if (increasing) std::reverse(inner.begin(), inner.end());
   radices.push_back(e);
   radices.insert(radices.end(), inner.begin(), inner.end());
   radices.push_back(e);

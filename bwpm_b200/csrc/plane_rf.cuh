@@ -35,6 +35,7 @@
 #pragma once
 
 #include <algorithm>
+#include <utility>
 #include <vector>
 
 #include "bulk.cuh"
@@ -613,28 +614,40 @@ inline RfRuntime<T> rf_runtime() {
   return {E, (const void*)k_cols_rf<Line>, (const void*)k_rows_rf<Line>};
 }
 
-// The run-time kernels of length n: the E (E² divides n, n/E threads per component and line) with
-// the smallest cost (equal_outer_plan), two lines per CTA where they fit. Lengths without such an E
-// keep the general kernels.
+// The run-time kernels of length n: of the E (E² divides n, n/E threads per component and line) from 4
+// on with 24 threads or more the one with the fewest stages, each an exchange of both lines and a
+// barrier, then the smallest cost (equal_outer_plan); else the other E with the smallest cost. Two lines
+// per CTA where they fit. Outer radices 2 and 3 cost rounding error (complex64 against the general
+// kernels, mean over facet and lens volumes, transmitted and reflected: E = 3 1.01, 1.02, E = 4 0.96,
+// 0.98, E = 6 0.95, 1.04, E = 8 and 10 0.97, 0.98; E = 2 up to 1.12) and threads (24 steps, ms: 500² FP64
+// 10·5·10 1.83, 2·5·5·5·2 2.43; 432² FP64 4·3·9·4 1.60, 3·8·6·3 1.72; 405² complex64 9·5·9 1.22, 3·9·5·3
+// 1.68); fewer threads leave latency (162² on 18 threads 10 % behind 54). Lengths without an E keep
+// the general kernels.
 template <typename T>
 inline RfKernels rf_pick_runtime(const std::vector<RfRuntime<T>>& all, int n) {
   RfKernels best;
-  double best_score = 1e29;
-  for (const RfRuntime<T>& c : all) {
-    if (2 * (n / c.e) > kRfThreads || n >= 1 << 15 || rf_smem<T>(n, 1, true) > 200 * 1024) continue;
-    const int nt = n / c.e;
-    std::vector<int> radices;
-    const double score = equal_outer_plan(n, c.e, nt, radices);
-    if (score >= best_score - 1e-9) continue;
-    best_score = score;
-    best.cols = c.cols;
-    best.rows = c.rows;
-    best.lines = 1;
-    if (4 * nt <= kRfThreads && rf_smem<T>(n, 2, true) <= 200 * 1024) best.lines = 2;
-    best.threads = (2 * best.lines * nt + 31) / 32 * 32;
-    best.cols_smem = rf_smem<T>(n, best.lines, true);
-    best.rows_smem = rf_smem<T>(n, best.lines, false);
-    best.radices = radices;
+  for (bool suits : {true, false}) {
+    std::pair<std::size_t, double> best_score{100, 1e29};
+    for (const RfRuntime<T>& c : all) {
+      if (2 * (n / c.e) > kRfThreads || n >= 1 << 15 || rf_smem<T>(n, 1, true) > 200 * 1024) continue;
+      const int nt = n / c.e;
+      if (suits != (c.e >= 4 && nt >= 24)) continue;
+      std::vector<int> radices;
+      const double cost = equal_outer_plan(n, c.e, nt, radices);
+      if (radices.empty()) continue;
+      const std::pair<std::size_t, double> score{suits ? radices.size() : 0, cost};
+      if (!(score < best_score)) continue;
+      best_score = score;
+      best.cols = c.cols;
+      best.rows = c.rows;
+      best.lines = 1;
+      if (4 * nt <= kRfThreads && rf_smem<T>(n, 2, true) <= 200 * 1024) best.lines = 2;
+      best.threads = (2 * best.lines * nt + 31) / 32 * 32;
+      best.cols_smem = rf_smem<T>(n, best.lines, true);
+      best.rows_smem = rf_smem<T>(n, best.lines, false);
+      best.radices = radices;
+    }
+    if (best.cols) return best;
   }
   return best;
 }
