@@ -267,19 +267,14 @@ __device__ __forceinline__ double r2f_flux(const cf (&v)[N / NT], const double* 
     c = (z - s) - y;
     s = z;
   }
-  // whole warps by shuffles, a partial last warp through shared memory
-  constexpr int NW = NT % 32 ? NT : NT / 32;
-  if constexpr (NT % 32 == 0) {
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if ((t & 31) == 0) red[t >> 5] = s;
-  } else {
-    red[t] = s;
-  }
+  static_assert(NT % 32 == 0, "whole warps");
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if ((t & 31) == 0) red[t >> 5] = s;
   __syncthreads();
   double total = 0.0;
   if (t == 0) {
     double comp = 0.0;
-    for (int i = 0; i < NW; ++i) {
+    for (int i = 0; i < NT / 32; ++i) {
       const double y = red[i] - comp;
       const double z = total + y;
       comp = (z - total) - y;
@@ -503,7 +498,7 @@ __global__ void __launch_bounds__(NT, MINB) k_resident2d_fixed(const R2Item* __r
   cf* S = b1 + rf::padded(N);
   float* mask_s = reinterpret_cast<float*>(smem_raw + lines_bytes(N, 3));
   __shared__ int s_item;
-  __shared__ double s_red[NT % 32 ? NT : NT / 32];
+  __shared__ double s_red[NT / 32];
   const int t = threadIdx.x;
   int phase = 0;
   for (;;) {
