@@ -4,7 +4,9 @@
 // multi-kernel form, mean over seeded δn volumes (transmitted, reflected): 512 points 0.98, 1.02 and
 // 1024 points 1.00, 0.90 (16 seeds, within their spread), 4096 points 1.00, 1.01 (96 seeds, ± 0.02).
 // On four CTAs (2048 points) it was 1.06, 1.00 and with run-time lengths (3000 points) 1.04, 1.08
-// (96 seeds, ± 0.02-0.03): those lengths, and the ones not measured, keep the multi-kernel form.
+// (96 seeds, ± 0.02-0.03): those lengths, and the ones not measured, keep the multi-kernel form. (At 2048
+// points both forms have the radices 8·8·8·4; a split line runs the inverse transform's C-point stage
+// first, the multi-kernel form last.)
 #include "born2d.cuh"
 
 namespace bwpm {

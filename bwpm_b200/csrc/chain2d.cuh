@@ -10,10 +10,12 @@
 // reflection gather), then the sparse sources; records of the next step load while the current
 // one computes, operator values are brought into L1 during the forward transform. A line on one SM
 // is bound by that SM's FP64 rate and issue from ≈ 1000 points on, so longer lines are split over
-// up to eight CTAs (cline.cuh), at an exchange of ≈ 0.7 µs per transform. Per step (200 slabs,
-// tilted facet and mask; launch per step → one CTA → split): FP64 256 points 10.5 → 1.4 µs, 1024
-// 17.3 → 3.1 → 2.7, 2430 44.4 → 13.7 → 6.9, 4096 41.1 → 15.9 → 5.3, 8192 129 → 9.9 (split);
-// complex64 1024 14.3 → 2.7, 2430 26.0 → 11.9 → 7.3, 4096 31.0 → 13.4 → 5.9.
+// up to eight CTAs (cline.cuh), at an exchange of ≈ 0.7 µs per transform. On split lines the
+// cluster-scope acquire of each exchange empties L1, so there the prefetch reaches L2 only: without it
+// steps with a mask are 2-4 % faster, steps that stay in the spectrum (below) 3-4 % slower (1024 and 1536
+// points, FP64). Per step (200 slabs, tilted facet and mask; launch per step → one CTA → split): FP64 256
+// points 10.5 → 1.4 µs, 1024 17.3 → 3.1 → 2.7, 2430 44.4 → 13.7 → 6.9, 4096 41.1 → 15.9 → 5.3, 8192
+// 129 → 9.9 (split); complex64 1024 14.3 → 2.7, 2430 26.0 → 11.9 → 7.3, 4096 31.0 → 13.4 → 5.9.
 //
 // A step that nothing acts on in real space (one pair, no mask, no sources to add, plane not
 // kept, not the last of its sweep) leaves its result in the spectrum: the inverse transform and

@@ -26,7 +26,7 @@
 //
 // Kernel times of a step (column + row kernel, mean over a lens or facet volume of 12 slabs, warm
 // caches), the kernels before → these: FP64 512² 37 + 32 → 12 + 13 µs, 375 × 250 32 + 49 → 15 + 11;
-// complex64 512² 9.8 + 12.5 → 9.4 + 10.6, 1024² 73 + 86 → 58 + 34. They issue on a third of the
+// complex64 512² 9.8 + 12.5 → 9.4 + 10.4, 1024² 73 + 86 → 58 + 32. They issue on a third of the
 // cycles; the rest waits on shared memory, barriers and the planes' loads. The prologue of each
 // kernel overlaps the end of the one before (programmatic dependent launch).
 //
